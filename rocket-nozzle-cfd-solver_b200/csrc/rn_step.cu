@@ -122,35 +122,19 @@ __device__ __forceinline__ int ext_prim(int e, int dx, int dy) {
   return T::NPT + e * 25 + (dy + 2) * 5 + (dx + 2);
 }
 
-// Faces of listed member e (slots NXF + NRF + 4e + w, w = W, E, S, N): the
-// face position, its direction, whether the reference draws it, and its
-// stencil as primitive slots (the 4 cells along the normal c0..c3, the 4
-// transverse sensor cells k1+t, k1-t, ij+t, ij-t).
-struct FaceSlot {
-  int c[4], s[4];
+// Position and direction of a listed member's face q = 4e + w (w = W, E, S, N;
+// slot NXF + NRF + q), and whether the reference draws it.
+struct FaceAt {
   int i, j;
   bool dirR, valid;
 };
-template <class T>
-__device__ __forceinline__ FaceSlot member_face_slot(int q, const int* xc, int Nx) {
-  FaceSlot f;
-  const int e = q >> 2, w = q & 3, m = xc[e];
-  const int mx = m % Nx, my = m / Nx;
-  if (w < 2) {
-    const int o = w;                             // face at mx + o
-    f.i = mx + o; f.j = my; f.dirR = false; f.valid = true;
-    f.c[0] = ext_prim<T>(e, o - 2, 0); f.c[1] = ext_prim<T>(e, o - 1, 0);
-    f.c[2] = ext_prim<T>(e, o, 0); f.c[3] = ext_prim<T>(e, o + 1, 0);
-    f.s[0] = ext_prim<T>(e, o - 1, 1); f.s[1] = ext_prim<T>(e, o - 1, -1);
-    f.s[2] = ext_prim<T>(e, o, 1); f.s[3] = ext_prim<T>(e, o, -1);
-  } else {
-    const int o = w - 2;                         // face at my + o
-    f.i = mx; f.j = my + o; f.dirR = true; f.valid = f.j != 0;
-    f.c[0] = ext_prim<T>(e, 0, o - 2); f.c[1] = ext_prim<T>(e, 0, o - 1);
-    f.c[2] = ext_prim<T>(e, 0, o); f.c[3] = ext_prim<T>(e, 0, o + 1);
-    f.s[0] = ext_prim<T>(e, 1, o - 1); f.s[1] = ext_prim<T>(e, -1, o - 1);
-    f.s[2] = ext_prim<T>(e, 1, o); f.s[3] = ext_prim<T>(e, -1, o);
-  }
+__device__ __forceinline__ FaceAt member_face_at(int q, const int* xc, int Nx) {
+  FaceAt f;
+  const int w = q & 3, m = xc[q >> 2];
+  f.dirR = w >= 2;
+  f.i = m % Nx + (f.dirR ? 0 : w);
+  f.j = m / Nx + (f.dirR ? w - 2 : 0);
+  f.valid = !f.dirR || f.j != 0;
   return f;
 }
 
@@ -210,9 +194,8 @@ __device__ __forceinline__ float rface_area(const Grid& g, int k, int x0, int y0
   const int ly = k / T::TX, lx = k - ly * T::TX, i = x0 + lx, j = y0 + ly;
   return (i < g.Nx && j <= g.Nr && j != 0) ? g.geoA[j * (g.Nx + 1) + i].w : 0.0f;
 }
-template <class T>
 __device__ __forceinline__ float member_face_area(const Grid& g, int q, const int* xc) {
-  const FaceSlot s = member_face_slot<T>(q, xc, g.Nx);
+  const FaceAt s = member_face_at(q, xc, g.Nx);
   if (!s.valid) return 0.0f;
   const float4* p = g.geoA + (s.j * (g.Nx + 1) + s.i);
   return s.dirR ? p->w : p->z;
@@ -334,7 +317,7 @@ __device__ __forceinline__ void load_prims(const Grid& g, const float4* __restri
       const float4 a = own ? R[k] : cells.a(i, j), b = own ? R[T::NPT8 + k] : cells.b(i, j);
       const bool solid = own ? sMask[ly * T::MW + mo + lx] != 0 : cells.solid(i, j);
       if (solid) {
-        W = make_float4(-1.0f, 0.0f, 0.0f, 1.0f);
+        W = wall_prim();
         Wb = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       } else {
         const Prim q = to_prim(a, b);
@@ -344,7 +327,7 @@ __device__ __forceinline__ void load_prims(const Grid& g, const float4* __restri
     } else if (i <= Nx + 1 && j <= Nr + 1) {
       ghost_prim_c(Nx, Nr, cells, i, j, t, P, W, Wb);
     } else {
-      W = make_float4(-1.f, 0.f, 0.f, 1.f); Wb = make_float4(0.f, 0.f, 0.f, 0.f);
+      W = wall_prim(); Wb = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     sW[k] = W;
     sWb[k] = Wb;
@@ -375,7 +358,7 @@ __device__ __forceinline__ void store_areas(const Grid& g, int x0, int y0, const
     for (int k = tid + T::NT; k < T::NXF; k += T::NT) sAr[k] = xface_area<T>(g, k, x0, y0);
   if constexpr (T::NRF > T::NT)
     for (int k = tid + T::NT; k < T::NRF; k += T::NT) sAr[T::NXF + k] = rface_area<T>(g, k, x0, y0);
-  for (int q = tid; q < 4 * xn; q += T::NT) sAr[T::NXF + T::NRF + q] = member_face_area<T>(g, q, xc);
+  for (int q = tid; q < 4 * xn; q += T::NT) sAr[T::NXF + T::NRF + q] = member_face_area(g, q, xc);
 }
 
 // FS_FLUX_X/R: every face of the tile (x-faces, then r-faces) and of its
@@ -411,7 +394,7 @@ __device__ __forceinline__ void inviscid_faces(const Grid& g, const rn_params& P
     const float area = sAr[k];   // the face's open area, 0 where it is not drawn
     if (area != 0.0f)
       f = face_flux(dirR, area, sW[b], sWb[b], sW[b + d], sWb[b + d], sW[b + 2 * d], sWb[b + 2 * d], sW[b + 3 * d],
-                    sWb[b + 3 * d], sW[b + d + t], sW[b + d - t], sW[b + 2 * d + t], sW[b + 2 * d - t], P);
+                    sWb[b + 3 * d], sW[b + d + t].w, sW[b + d - t].w, sW[b + 2 * d + t].w, sW[b + 2 * d - t].w, P);
     sF[k] = f.F; sY[k] = f.Y; sO[k] = f.O;
   }
 }
@@ -453,8 +436,8 @@ __device__ __forceinline__ void group_flux(int Hx, int Hy, int sm_, int x0, int 
 template <class T, int STAGE>
 __device__ __forceinline__ bool update_cell(const StageArgs& a, const CellSrc<T>& cs, const rn_params& P, int i,
                                             int j, float dt, float t, int x0, int y0, const int* xc, int xn,
-                                            const float4* sF, const float4* sY, const float* sO, const float* sAr,
-                                            float4& oA, float4& oB) {
+                                            const float4* sW, const float4* sWb, const float4* sF, const float4* sY,
+                                            const float* sO, const float* sAr, float4& oA, float4& oB) {
   const Grid& g = a.g;
   const int Nx = g.Nx;
   const int k = j * Nx + i;
@@ -475,7 +458,13 @@ __device__ __forceinline__ bool update_cell(const StageArgs& a, const CellSrc<T>
     if (STAGE == 2) { A0 = a.A0[kh]; B0 = a.B0[kh]; }
     ghz = cs.gm(Hx, Hy).z;
   }
-  Prim q = to_prim(A, B);
+  // the host's primitives: it lies within a cell of the tile, so the primitive
+  // phase left them in its halo slot (the same floats as to_prim's)
+  const int hs = (Hy - y0 + 2) * T::PX + (Hx - x0 + 2);
+  Prim q;
+  q.w = sW[hs];
+  q.s = sWb[hs];
+  if (q.w.x < 0.0f) q = to_prim(A, B);         // a solid host
   float4 L = make_float4(0.f, 0.f, 0.f, 0.f), LY = L;
   float LO = 0.0f;
   const int sm_ = iround(ghz);
@@ -507,8 +496,13 @@ __device__ __forceinline__ bool update_cell(const StageArgs& a, const CellSrc<T>
   float rho = fmaxf(U.x, RHO_MIN);
   const Over per_den = over(fmaxf(U.x, RHO_MIN));
   float vx = per_den(U.y), vy = per_den(U.z);
+#ifdef RN_FAST
+  const float sp2 = vx * vx + vy * vy;         // the speed itself only where it is above the cap
+  if (sp2 > P.vMax * P.vMax) { float s = P.vMax * rsqrtf(sp2); vx *= s; vy *= s; }
+#else
   float sp = len2(vx, vy);
   if (sp > P.vMax) { float s = fdiv(P.vMax, sp); vx *= s; vy *= s; }
+#endif
   if (!(rho < 1e30f) || !(vx < 1e30f && vx > -1e30f)) {   // NaN guard
     oA = make_float4(P.ambCons[0], P.ambCons[1], P.ambCons[2], P.ambCons[3]);
     oB = make_float4(P.ambB[0], P.ambB[1], P.ambB[2], P.ambB[3]);
@@ -585,7 +579,7 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
   float wcell = 0.0f;
   if (tid < T::NC && i < Nx && j < Nr) {
     float4 oA, oB;
-    const bool fluid = update_cell<T, STAGE>(a, cs, P, i, j, dt, t, x0, y0, xc, xn, sF, sY, sO, sAr, oA, oB);
+    const bool fluid = update_cell<T, STAGE>(a, cs, P, i, j, dt, t, x0, y0, xc, xn, sW, sWb, sF, sY, sO, sAr, oA, oB);
     const int k = j * Nx + i;
     a.oA[k] = oA;
     a.oB[k] = oB;
@@ -869,7 +863,7 @@ __device__ __forceinline__ void stage2_physics_body(const StageArgs& a, const Ph
         else { const int m = xc[q - T::NC]; i = m % Nx; j = m / Nx; }
         if (i < Nx && j < Nr) {
           float4 oA, oB;
-          update_cell<T, 2>(a, cs, P, i, j, dt, t, x0, y0, xc, xn, sF, sY, sO, sAr, oA, oB);
+          update_cell<T, 2>(a, cs, P, i, j, dt, t, x0, y0, xc, xn, sW, sWb, sF, sY, sO, sAr, oA, oB);
           sA2[q] = oA;
           sB2[q] = oB;
         }
