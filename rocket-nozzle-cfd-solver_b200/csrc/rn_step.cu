@@ -712,8 +712,19 @@ __device__ __forceinline__ bool source_cell(const Grid& g, const CellSrc<T>& cs,
       float rs = fdiv(p, Rm * Ts), mus = sutherland(Ts * P.gas[2], P);
       float dz = 2.0f * clampf(fdiv(0.5f * V, wl), 0.25f, 1.0f);
       float nz = fdiv(mus, rs * dz);
-      float tw = up <= 69.7f * nz ? fdiv(2.0f * mus * up, dz)
-                                  : rs * powf(7.187f * powf(nz, 1.142857f) + 0.13769f * powf(nz, 0.142857f) * up, 1.75f);
+      // turbulent branch rs (7.187 nz^(8/7) + 0.13769 nz^(1/7) up)^(7/4)
+      float turb;
+#ifdef RN_FAST
+      // nz^(8/7) = nz nz^(1/7) and x^(7/4) = x sqrt(x) sqrt(sqrt(x)): one powf
+      // where the reference's three take most of a wall cell's time (the
+      // slowest threads of the split step)
+      const float n7 = powf(nz, 0.142857f);
+      const float x = n7 * (7.187f * nz + 0.13769f * up), x2 = sqrtf(x);
+      turb = rs * x * x2 * sqrtf(x2);
+#else
+      turb = rs * powf(7.187f * powf(nz, 1.142857f) + 0.13769f * powf(nz, 0.142857f) * up, 1.75f);
+#endif
+      float tw = up <= 69.7f * nz ? fdiv(2.0f * mus * up, dz) : turb;
       tw = fminf(tw, fdiv(0.3f * rho * up * V, fmaxf(wl * dt, 1e-9f)));
       if (up > 1e-6f) { L.y -= fdiv(tw * wl * utx, up); L.z -= fdiv(tw * wl * uty, up); }
       float qw = fdiv(tw, fmaxf(up, 1e-4f)) * cp * (Taw - P.Tw) * 1.24f;
@@ -1166,19 +1177,22 @@ static dim3 tiles_of(const Grid& g) {
   return dim3((g.Nx + T::TX - 1) / T::TX, (g.Nr + T::TY - 1) / T::TY);
 }
 
+// A step kernel's dynamic shared-memory limit, and the SM's whole L1/shared
+// array as shared memory: consecutive kernels of a step then ask for the same
+// split, which an SM could only change between kernels while idle.
+template <class K>
+static bool step_kernel_attributes(K* kernel, size_t smem) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) == cudaSuccess &&
+         cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                              cudaSharedmemCarveoutMaxShared) == cudaSuccess;
+}
 template <class T>
 static int init_tile() {
-  const int ss = int(stage_smem_t<T>(MAXX)), ps = int(fused_smem_t<T>(MAXX));
-  if (cudaFuncSetAttribute(k_stage<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) != cudaSuccess) return -1;
-  if (cudaFuncSetAttribute(k_stage<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) != cudaSuccess) return -1;
-  if (cudaFuncSetAttribute(k_stage2phys<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, ps) != cudaSuccess) return -1;
-  if (cudaFuncSetAttribute(k_stage_batch<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) != cudaSuccess)
-    return -1;
-  if (cudaFuncSetAttribute(k_stage_batch<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) != cudaSuccess)
-    return -1;
-  if (cudaFuncSetAttribute(k_stage2phys_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, ps) != cudaSuccess)
-    return -1;
-  return 0;
+  const size_t ss = stage_smem_t<T>(MAXX), ps = fused_smem_t<T>(MAXX);
+  const bool ok = step_kernel_attributes(k_stage<T, 1>, ss) && step_kernel_attributes(k_stage<T, 2>, ss) &&
+                  step_kernel_attributes(k_stage2phys<T>, ps) && step_kernel_attributes(k_stage_batch<T, 1>, ss) &&
+                  step_kernel_attributes(k_stage_batch<T, 2>, ss) && step_kernel_attributes(k_stage2phys_batch<T>, ps);
+  return ok ? 0 : -1;
 }
 // Raises the dynamic shared-memory limits of the stage and physics kernels to
 // what a member list of MAXX cells needs (process-wide function attributes).
