@@ -114,11 +114,11 @@ int rn_set_state(rn_handle h, const float* A, const float* B);
 /* readAll() (solver.js:1075) */
 int rn_get_state(rn_handle h, float* A, float* B);
 /* step(n, P) (solver.js:849-891), including GPUSpray.step (spray.js:256-297)
- * when P->inj is set: queued on the handle's stream. For n of two periods or
- * more (12 steps, 4 with sprays) the handle captures one period of its
- * launches into a CUDA graph and replays it (the same kernels, the same
- * bits); not while profiling, and not while the caller is itself capturing
- * the handle's stream. */
+ * when P->inj is set: queued on the handle's stream. For n of 12 or more (4
+ * with sprays, or when the same call came just before) the handle captures an
+ * even number of its steps into a CUDA graph and replays it (the same kernels,
+ * the same bits); not while profiling, and not while the caller is itself
+ * capturing the handle's stream. */
 int rn_step(rn_handle h, int n, const rn_params* P);
 /* rescaleAmbient(fp, fT, du, P) (solver.js:998-1010) */
 int rn_rescale_ambient(rn_handle h, float fp, float fT, float du, const rn_params* P);
@@ -218,7 +218,7 @@ int rn_autotune(rn_handle h, const rn_params* P, int steps, int* chosen);
  * launch per kernel kind per step: every tile of every member is a block of
  * the same grid. Members must share the physics flags (visc, chem, inj) and
  * the precision; each keeps its own state, geometry, dt and parameter block.
- * rn_batch_step captures the periodic 6-step launch sequence in a CUDA graph
+ * rn_batch_step captures 6 steps of its launch sequence in a CUDA graph
  * and replays it. While in a batch a handle must not be stepped on its own;
  * all other handle calls (reads, integrals) work between batch steps.
  * Removing a member leaves its handle where the batch left it. */

@@ -47,11 +47,17 @@ constexpr int SPRAY_N = 65536;
 int rn_record_error(int code, const std::string& msg) { return fail(code, msg); }
 int rn_record_cuda(cudaError_t e, const char* what) { return cuda_fail(e, what); }
 
+void rn_drop_step_graphs(rn_solver* h) {
+  for (StepGraph& g : h->graphs) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
+  }
+}
+
 namespace {
 
 void free_buffers(rn_solver* h) {
-  if (h->stepGraph) cudaGraphExecDestroy(h->stepGraph);   // its launches name these buffers
-  h->stepGraph = nullptr;
+  rn_drop_step_graphs(h);   // their launches name these buffers
   cudaFree(h->SA[0]);   // base of the 6-plane state ring
   for (int s = 0; s < 3; s++) h->SA[s] = h->SB[s] = nullptr;
   cudaFree(h->geoA); cudaFree(h->geoG); cudaFree(h->geoM); cudaFree(h->jw); cudaFree(h->wallRow);
@@ -257,8 +263,7 @@ int rn_mask_refresh(rn_solver* h) {
 // inside it (a sliver merged across the tile edge). Groups are a host plus the
 // slaves of its slave mask (geoM.z bits 1/2/4/8, cutcell.js:168-174).
 int rn_build_member_lists(rn_solver* h) {
-  if (h->stepGraph) cudaGraphExecDestroy(h->stepGraph);   // its launches name the old lists
-  h->stepGraph = nullptr;
+  rn_drop_step_graphs(h);   // their launches name the old lists
   const int TX = TILE_TX[h->tile], TY = TILE_TY[h->tile];
   const int Nx = h->Nx, Nr = h->Nr, tx = (Nx + TX - 1) / TX, nT = tx * ((Nr + TY - 1) / TY);
   const uint8_t* mask = h->hostMask.data();
@@ -558,13 +563,15 @@ int rn_get_state(rn_handle h, float* A, float* B) {
 }  // extern "C"
 
 namespace {
-constexpr int STEP_PERIOD = 6;   // 3 ring shifts x 2 step-info parities
+constexpr int STEP_PERIOD = 2;   // the launches of a step depend on the step-info parity (ring_slots)
 
 // One time step of handle h (the body of step(n, P), solver.js:849-891).
 int step_once(rn_solver* h, const rn_params* P) {
   const Grid g = h->grid();
   const bool phys = P->visc || P->chem, inj = P->inj != 0;
-  const int s0 = h->cur, s1 = (h->cur + 1) % 3, s2 = (h->cur + 2) % 3;
+  const int s0 = h->cur;
+  int s1, s2;
+  ring_slots(s0, h->stepIdx, s1, s2);
   unsigned* wIn = h->wmax + h->wslot;
   unsigned* wOut = h->wmax + (1 - h->wslot);
   if (!h->wvalid) {
@@ -665,7 +672,7 @@ int step_once(rn_solver* h, const rn_params* P) {
   h->cur = s2;
   if (inj) {
     if (!h->prof) CK(cudaStreamWaitEvent(h->stream, h->evSprayJoin, 0));   // the parcel step is done
-    const int out = (h->cur + 1) % 3;
+    const int out = s0;                       // the step's base state, read by now
     ApplyArgs ap;
     ap.g = g;
     ap.A = h->SA[h->cur]; ap.B = h->SB[h->cur]; ap.src = h->src;
@@ -693,16 +700,83 @@ int step_once(rn_solver* h, const rn_params* P) {
   return RN_OK;
 }
 
-// Whether the handle's 6-step graph can replay the next steps with P: the
-// kernels, launch shapes, buffers and parameter block it was captured with.
-bool graph_matches(const rn_solver* h, const rn_params* P) {
-  return h->stepGraph && h->graphK == h->K && h->graphTile == h->tile && h->graphMaxX == h->maxX &&
-         h->graphHeavy == h->nHeavy && h->graphBase == h->SA[0] && h->graphXoff == h->xoff &&
-         std::memcmp(&h->graphP, P, sizeof(rn_params)) == 0;
+// Whether graph g replays the handle's next steps with P: captured with the
+// kernels, launch shapes, buffers and parameter block that hold now, from the
+// ring position the handle is at (up to one step of the two-step period).
+bool graph_matches(const rn_solver* h, const StepGraph& g, const rn_params* P) {
+  return g.exec && g.K == h->K && g.tile == h->tile && g.maxX == h->maxX && g.nHeavy == h->nHeavy &&
+         g.base == h->SA[0] && g.xoff == h->xoff && std::memcmp(&g.P, P, sizeof(rn_params)) == 0;
 }
-void drop_step_graph(rn_solver* h) {
-  if (h->stepGraph) cudaGraphExecDestroy(h->stepGraph);
-  h->stepGraph = nullptr;
+bool graph_at_start(const rn_solver* h, const StepGraph& g, bool inj) {
+  return h->cur == g.cur && h->stepIdx == g.stepIdx && h->wslot == g.wslot && (!inj || h->scur == g.scur);
+}
+
+// Relative cost of n steps through a graph of B steps: each replay (about 3 us
+// on the device between two graphs, measured), each remaining step launched
+// kernel by kernel (4 us of the host a kernel), and a share of instantiating
+// the graph's nodes. k = kernels per step.
+double graph_cost(int n, int B, int k) { return (n / B) * 3.0 + (n % B) * 4.0 * k + 2.0 * B * k; }
+constexpr int GRAPH_NODES = 24;   // most kernels captured in one graph
+int graph_steps(int n, int k) {
+  int best = STEP_PERIOD;
+  for (int B = STEP_PERIOD; B <= n && B * k <= GRAPH_NODES; B += STEP_PERIOD)
+    if (graph_cost(n, B, k) < graph_cost(n, best, k)) best = B;
+  return best;
+}
+
+// Streams that the captured launches fork to exist before the capture.
+int ready_side_streams(rn_solver* h, bool inj) {
+  if (h->nHeavy > 0 && !h->side) {
+    CK(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&h->evFork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&h->evJoin, cudaEventDisableTiming));
+  }
+  if (inj && !h->sprayStream) {
+    CK(cudaStreamCreateWithFlags(&h->sprayStream, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&h->evSprayFork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&h->evSprayJoin, cudaEventDisableTiming));
+  }
+  return RN_OK;
+}
+
+// Captures the next B steps of h into slot g.
+int capture_steps(rn_solver* h, const rn_params* P, int B, StepGraph& g) {
+  const bool inj = P->inj != 0;
+  if (g.exec) cudaGraphExecDestroy(g.exec);
+  g.exec = nullptr;
+  int rc = ready_side_streams(h, inj);
+  if (rc != RN_OK) return rc;
+  const int cur = h->cur, stepIdx = h->stepIdx, wslot = h->wslot, s1last = h->s1last, scur = h->scur;
+  const uint32_t head = h->head, seed = h->seed;
+  const long long stepCount = h->stepCount, launches = h->launches;
+  cudaGraph_t gr = nullptr;
+  h->hsOnDevice = inj;
+  cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) {
+    for (int k = 0; k < B && rc == RN_OK; k++) rc = step_once(h, P);
+    e = cudaStreamEndCapture(h->stream, &gr);
+  }
+  h->hsOnDevice = false;
+  g.launches = h->launches - launches;
+  h->cur = cur; h->stepIdx = stepIdx; h->wslot = wslot; h->s1last = s1last; h->scur = scur;
+  h->head = head; h->seed = seed;
+  h->stepCount = stepCount; h->launches = launches;
+  if (rc == RN_OK && e != cudaSuccess) rc = cuda_fail(e, "rn_step: graph capture");
+  if (rc == RN_OK) {
+    e = cudaGraphInstantiate(&g.exec, gr, 0);
+    if (e != cudaSuccess) {
+      g.exec = nullptr;
+      rc = cuda_fail(e, "rn_step: graph instantiate");
+    }
+  }
+  if (gr) cudaGraphDestroy(gr);
+  if (rc != RN_OK) return rc;
+  g.K = h->K; g.base = h->SA[0]; g.xoff = h->xoff;
+  g.tile = h->tile; g.maxX = h->maxX; g.nHeavy = h->nHeavy;
+  g.cur = cur; g.stepIdx = stepIdx; g.wslot = wslot; g.scur = scur;
+  g.steps = B;
+  g.P = *P;
+  return RN_OK;
 }
 
 // Profiling inside graph replays (rn_profile mode 2, steps without sprays):
@@ -711,17 +785,26 @@ void drop_step_graph(rn_solver* h) {
 // period, the pairs read after each replay, so each kernel is timed as it
 // runs in the replayed graph (no host launch gaps between the kernels). The
 // steps before the first whole period run one by one, timed launch by launch.
+constexpr int PROF_STEPS = 6;   // a multiple of STEP_PERIOD
+// Slot of the stage-1 state after an even number of steps from here: that of
+// the step before (cur, stepIdx).
+int last_s1(const rn_solver* h, bool inj) {
+  int s1, s2;
+  ring_slots(h->cur, h->stepIdx, s1, s2);
+  // without sprays both steps of a period use the same stage-1 slot; with
+  // them cur stays and the other parity's slot was the last one
+  return inj ? s2 : s1;
+}
 int prof_graph_steps(rn_solver* h, const rn_params* P, int n, int& done) {
   while (done < n && !h->wvalid) {
     int rc = step_once(h, P);
     if (rc != RN_OK) return rc;
     done++;
   }
-  if (n - done < STEP_PERIOD) return RN_OK;
-  if (h->nHeavy > 0 && !h->side) {   // the helper stream exists before the capture
-    CK(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&h->evFork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&h->evJoin, cudaEventDisableTiming));
+  if (n - done < PROF_STEPS) return RN_OK;
+  {
+    const int rc = ready_side_streams(h, false);
+    if (rc != RN_OK) return rc;
   }
   const int cur = h->cur, stepIdx = h->stepIdx, wslot = h->wslot, s1last = h->s1last;
   const long long stepCount = h->stepCount, launches = h->launches;
@@ -731,7 +814,7 @@ int prof_graph_steps(rn_solver* h, const rn_params* P, int n, int& done) {
   h->profCapture = true;
   cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
   int rc = RN_OK;
-  for (int k = 0; k < STEP_PERIOD && rc == RN_OK && e == cudaSuccess; k++) rc = step_once(h, P);
+  for (int k = 0; k < PROF_STEPS && rc == RN_OK && e == cudaSuccess; k++) rc = step_once(h, P);
   cudaError_t e2 = e == cudaSuccess ? cudaStreamEndCapture(h->stream, &gr) : e;
   h->profCapture = false;
   const long long perPeriod = h->launches - launches;
@@ -750,7 +833,7 @@ int prof_graph_steps(rn_solver* h, const rn_params* P, int n, int& done) {
   if (e2 != cudaSuccess) { release(); return cuda_fail(e2, "rn_step: profiled graph capture"); }
   e = cudaGraphInstantiate(&ex, gr, 0);
   if (e != cudaSuccess) { ex = nullptr; release(); return cuda_fail(e, "rn_step: profiled graph instantiate"); }
-  while (n - done >= STEP_PERIOD) {
+  while (n - done >= PROF_STEPS) {
     e = cudaGraphLaunch(ex, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     for (auto& p : h->profGraphEv) {
@@ -760,10 +843,10 @@ int prof_graph_steps(rn_solver* h, const rn_params* P, int n, int& done) {
       h->profN[p.first] += 1;
     }
     if (e != cudaSuccess) { release(); return cuda_fail(e, "rn_step: profiled graph replay"); }
-    h->s1last = (h->cur + 1 + 2 * (STEP_PERIOD - 1)) % 3;
-    h->stepCount += STEP_PERIOD;
+    h->s1last = last_s1(h, false);
+    h->stepCount += PROF_STEPS;
     h->launches += perPeriod;
-    done += STEP_PERIOD;
+    done += PROF_STEPS;
   }
   release();
   return RN_OK;
@@ -782,84 +865,66 @@ int rn_step(rn_handle h, int n, const rn_params* P) {
   if (h->batch) return fail(RN_ERR_STATE, "rn_step: the handle is stepped by a batch");
   const bool inj = P->inj != 0;
   int done = 0;
-  // The launch sequence repeats: every 6 steps without sprays (3 ring shifts x
-  // 2 step-info parities), every 2 with them (the state ring stays put, the
-  // step info, wave-speed slot and parcel ring alternate; the ring head and
-  // seed are then read and advanced on the device). Whole periods replay from
-  // a CUDA graph captured from the handle's own launches (not while
-  // profiling, which brackets each kernel with events).
-  const int period = inj ? 2 : STEP_PERIOD;
-  auto at_start = [&]() {
-    return h->cur == h->graphCur && h->stepIdx == h->graphStepIdx && h->wslot == h->graphWslot &&
-           (!inj || h->scur == h->graphScur);
-  };
-  // (nor when the caller is capturing the handle's stream into a graph of its
-  // own: the launches then go into that graph as they are)
+  // The launch sequence repeats every two steps (the state ring, step info,
+  // wave-speed slot and parcel ring alternate; the spray's ring head and seed
+  // are read and advanced on the device). Runs of steps replay from a CUDA
+  // graph captured from the handle's own launches (not while profiling, which
+  // brackets each kernel with events, nor when the caller is capturing the
+  // handle's stream into a graph of its own: the launches then go into that
+  // graph as they are).
+  const int perStep = 2 + (inj ? 2 : 0);
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cs = cudaStreamCaptureStatusNone;
-  if (h->prof == 2 && !inj && cs == cudaStreamCaptureStatusNone && n >= 2 * period) {
+  if (h->prof == 2 && !inj && cs == cudaStreamCaptureStatusNone && n >= 2 * PROF_STEPS) {
     int rc = prof_graph_steps(h, P, n, done);
     if (rc != RN_OK) return rc;
   }
-  if (!h->prof && cs == cudaStreamCaptureStatusNone && n >= 2 * period) {
-    while (done < n && (!h->wvalid || (graph_matches(h, P) && !at_start()))) {
-      int rc = step_once(h, P);
+  // a graph pays within one call from about 12 steps on; shorter calls get one
+  // when the same call comes a second time
+  const bool again = h->lastN == n && std::memcmp(&h->lastP, P, sizeof(rn_params)) == 0;
+  h->lastN = n;
+  h->lastP = *P;
+  if (!h->prof && cs == cudaStreamCaptureStatusNone && n >= 2 * STEP_PERIOD && (n >= 12 || inj || again)) {
+    int rc = rn_ensure_wave_speed(h);
+    if (rc != RN_OK) return rc;
+    const int want = graph_steps(n, perStep);
+    StepGraph* g = nullptr;
+    for (StepGraph& q : h->graphs)
+      if (graph_matches(h, q, P) && q.steps <= n && (!g || q.steps == want)) g = &q;
+    // a graph of another length serves too unless it is much the worse one
+    if (g && graph_cost(n, g->steps, perStep) > 1.25 * graph_cost(n, want, perStep) + 10.0) g = nullptr;
+    if (!g) {
+      g = &h->graphs[h->graphs[1].used < h->graphs[0].used ? 1 : 0];
+      rc = capture_steps(h, P, want, *g);
+      if (rc != RN_OK) return rc;
+    }
+    g->used = ++h->graphClock;
+    if (!graph_at_start(h, *g, inj)) {          // the other parity (or another ring position)
+      rc = step_once(h, P);
       if (rc != RN_OK) return rc;
       done++;
-    }
-    if (n - done >= period && !graph_matches(h, P)) {
-      drop_step_graph(h);
-      if (h->nHeavy > 0 && !h->side) {   // the helper streams exist before the capture
-        CK(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&h->evFork, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&h->evJoin, cudaEventDisableTiming));
+      if (!graph_at_start(h, *g, inj) && n - done >= g->steps) {
+        rc = capture_steps(h, P, g->steps, *g);
+        if (rc != RN_OK) return rc;
       }
-      if (inj && !h->sprayStream) {
-        CK(cudaStreamCreateWithFlags(&h->sprayStream, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&h->evSprayFork, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&h->evSprayJoin, cudaEventDisableTiming));
-      }
-      const int cur = h->cur, stepIdx = h->stepIdx, wslot = h->wslot, s1last = h->s1last, scur = h->scur;
-      const uint32_t head = h->head, seed = h->seed;
-      const long long stepCount = h->stepCount, launches = h->launches;
-      cudaGraph_t gr = nullptr;
-      h->hsOnDevice = inj;
-      CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-      int rc = RN_OK;
-      for (int k = 0; k < period && rc == RN_OK; k++) rc = step_once(h, P);
-      cudaError_t e = cudaStreamEndCapture(h->stream, &gr);
-      h->hsOnDevice = false;
-      const long long perPeriod = h->launches - launches;
-      h->cur = cur; h->stepIdx = stepIdx; h->wslot = wslot; h->s1last = s1last; h->scur = scur;
-      h->head = head; h->seed = seed;
-      h->stepCount = stepCount; h->launches = launches;
-      if (rc != RN_OK) { if (gr) cudaGraphDestroy(gr); return rc; }
-      if (e != cudaSuccess) { if (gr) cudaGraphDestroy(gr); return cuda_fail(e, "rn_step: graph capture"); }
-      e = cudaGraphInstantiate(&h->stepGraph, gr, 0);
-      cudaGraphDestroy(gr);
-      if (e != cudaSuccess) { h->stepGraph = nullptr; return cuda_fail(e, "rn_step: graph instantiate"); }
-      h->graphK = h->K; h->graphTile = h->tile; h->graphMaxX = h->maxX; h->graphHeavy = h->nHeavy;
-      h->graphBase = h->SA[0]; h->graphXoff = h->xoff; h->graphP = *P;
-      h->graphCur = cur; h->graphStepIdx = stepIdx; h->graphWslot = wslot; h->graphScur = scur;
-      h->graphLaunches = perPeriod;
-      h->graphPeriod = period;
     }
-    if (graph_matches(h, P) && h->graphPeriod == period && h->wvalid && at_start() && n - done >= period) {
+    if (graph_at_start(h, *g, inj) && n - done >= g->steps) {
       if (inj) {   // the ring head and seed the graph's parcel kernels read
         k_set_hs<<<1, 1, 0, h->stream>>>(h->dHS, h->head, h->seed);
         h->launches++;
       }
-      while (n - done >= period) {
-        CK(cudaGraphLaunch(h->stepGraph, h->stream));
-        // a period leaves the rings, step info and wave-speed slot where they were
-        h->s1last = inj ? (h->cur + 1) % 3 : (h->cur + 1 + 2 * (period - 1)) % 3;
+      while (n - done >= g->steps) {
+        CK(cudaGraphLaunch(g->exec, h->stream));
+        // an even number of steps leaves the rings, step info and wave-speed
+        // slot where they were
+        h->s1last = last_s1(h, inj);
         if (inj) {
-          h->head = (h->head + 4u * uint32_t(period)) % SPRAY_N;
-          h->seed = h->seed + uint32_t(period);
+          h->head = (h->head + 4u * uint32_t(g->steps)) % SPRAY_N;
+          h->seed = h->seed + uint32_t(g->steps);
         }
-        h->stepCount += period;
-        h->launches += h->graphLaunches;
-        done += period;
+        h->stepCount += g->steps;
+        h->launches += g->launches;
+        done += g->steps;
       }
     }
   }

@@ -11,8 +11,8 @@
 // descriptor (BatchInst: buffers, ring position, parameter block) in a device
 // array. The descriptor's ring position is normalised to the batch's step
 // counter, so it stays the same from call to call while the members are only
-// stepped by the batch, and the launch sequence repeats with a period of 6
-// steps (3 ring shifts x 2 step-info parities). Without sprays that period is
+// stepped by the batch, and the launch sequence repeats with a period of two
+// steps (the two step-info parities). Without sprays a few periods are
 // captured once in a CUDA graph and replayed.
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -25,16 +25,13 @@
 using namespace rn;
 
 namespace {
-constexpr int PERIOD = 6;
+constexpr int PERIOD = 2;        // a step's launches depend on the step-info parity (batch_ring)
+constexpr int GRAPH_STEPS = 6;   // steps captured in the batch's graph, a multiple of PERIOD
 constexpr int SPRAY_N = 65536;
 
 struct Flags {
   int visc = 0, chem = 0, inj = 0;
   bool phys() const { return visc || chem; }
-  // how far the state ring turns per step (rn_step's slot bookkeeping): the
-  // step's kernels write s1, then s2 (stage 2, or stage 2 fused with the
-  // split step); the spray apply writes the slot after s2
-  int delta() const { return inj ? 0 : 2; }
   bool operator==(const Flags& o) const { return visc == o.visc && chem == o.chem && inj == o.inj; }
 };
 Flags flags_of(const rn_params& P) {
@@ -119,12 +116,13 @@ int index_of(const rn_batch_t* b, const rn_solver* h) {
 }
 
 // Normalised ring position of member h at batch step counter ctr: the kernels
-// of batch step c use slot (cur0 + c*delta) % 3 and parity stepIdx0 ^ (c & 1).
+// of batch step c find its ring slots through batch_ring at parity c & 1.
 void normalise(const rn_batch_t* b, const rn_solver* h, int& cur0, int& si0, int& ws0) {
-  const int sh = (b->ctr * b->flags.delta()) % 3, par = b->ctr & 1;
-  cur0 = (h->cur - sh + 3) % 3;
+  const int par = b->ctr & 1;
   si0 = h->stepIdx ^ par;
   ws0 = h->wslot ^ par;
+  // at odd parity without sprays the ring has turned by 2 d0 = -d0 (mod 3)
+  cur0 = par && !b->flags.inj ? (h->cur + (si0 ? 2 : 1)) % 3 : h->cur;
 }
 
 // Brings the block table, the descriptors on the device and the members'
@@ -248,10 +246,9 @@ int refresh(rn_batch_t* b) {
 // With sprays, the per-member parcel and apply launches go between them.
 int launch_step(rn_batch_t* b, int c, bool withSpray) {
   const Flags f = b->flags;
-  const int delta = f.delta();
   BatchPhase ph;
-  ph.shift = (c * delta) % 3;
   ph.par = c & 1;
+  ph.turn = ph.par && !f.inj;
   ph.maxX = b->maxX;
   ph.active = b->runActive.empty() ? nullptr : b->dActive;
   const int nb = b->nblocks;
@@ -274,7 +271,8 @@ int launch_step(rn_batch_t* b, int c, bool withSpray) {
       if (!b->runActive.empty() && !b->runActive[m]) continue;   // stopped in rn_batch_run
       rn_solver* h = b->members[m];
       const BatchInst& d = b->uploaded[m];
-      const int s0 = (d.cur0 + ph.shift) % 3, s1 = (s0 + 1) % 3;
+      int s0, s1, s2;
+      batch_ring(d, ph, s0, s1, s2);
       const int si = d.stepIdx0 ^ ph.par;
       SprayArgs sp;
       sp.g = h->grid();
@@ -322,8 +320,9 @@ int launch_step(rn_batch_t* b, int c, bool withSpray) {
       if (!b->runActive.empty() && !b->runActive[m]) continue;
       rn_solver* h = b->members[m];
       const BatchInst& d = b->uploaded[m];
-      const int s0 = (d.cur0 + ph.shift) % 3;
-      const int cur = (s0 + 2) % 3, out = (cur + 1) % 3;
+      int s0, s1, s2;
+      batch_ring(d, ph, s0, s1, s2);
+      const int cur = s2, out = s0;
       const int ws = d.wslot0 ^ ph.par;
       ApplyArgs ap;
       ap.g = h->grid();
@@ -351,7 +350,7 @@ int build_graph(rn_batch_t* b) {
   BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   const long long before = b->launches;
   int rc = RN_OK;
-  for (int c = 0; c < PERIOD && rc == RN_OK; c++) rc = launch_step(b, c, false);
+  for (int c = 0; c < GRAPH_STEPS && rc == RN_OK; c++) rc = launch_step(b, c, false);
   cudaError_t e = cudaStreamEndCapture(b->stream, &g);
   b->launches = before;   // capturing launches nothing
   if (rc != RN_OK) {
@@ -379,7 +378,7 @@ int launches_per_step(const rn_batch_t* b) { return 2 + ((b->flags.phys() && b->
 
 // The launches of n batch steps from the batch counter on (descriptors and
 // block table already refreshed): without sprays, up to the start of a period
-// step by step, whole periods from the graph, the rest step by step.
+// step by step, runs of GRAPH_STEPS from the graph, the rest step by step.
 int issue_steps(rn_batch_t* b, int n) {
   int done = 0, rc = RN_OK;
   if (b->flags.inj) {
@@ -397,7 +396,7 @@ int issue_steps(rn_batch_t* b, int n) {
     b->ctr = (b->ctr + 1) % PERIOD;
     done++;
   }
-  if (n - done >= PERIOD) {
+  if (n - done >= GRAPH_STEPS) {
     const int* active = b->runActive.empty() ? nullptr : b->dActive;
     if (!b->graph || b->graphK != b->K || b->graphBlocks != b->nblocks || b->graphTile != b->tile ||
         b->graphMaxX != b->maxX || b->graphHeavy != (b->split ? b->nHeavy : 0) || !(b->graphFlags == b->flags) ||
@@ -405,10 +404,10 @@ int issue_steps(rn_batch_t* b, int n) {
       rc = build_graph(b);
       if (rc != RN_OK) return rc;
     }
-    while (n - done >= PERIOD) {
+    while (n - done >= GRAPH_STEPS) {
       BCK(cudaGraphLaunch(b->graph, b->stream));
-      b->launches += PERIOD * launches_per_step(b);
-      done += PERIOD;
+      b->launches += GRAPH_STEPS * launches_per_step(b);
+      done += GRAPH_STEPS;
     }
   }
   for (; done < n; done++) {
@@ -422,13 +421,19 @@ int issue_steps(rn_batch_t* b, int n) {
 // A member's host-side bookkeeping after n batch steps, as n calls of rn_step
 // would leave it.
 void advance(rn_solver* h, long long n, const Flags& f) {
-  h->cur = int((h->cur + n * f.delta()) % 3);
+  if (n <= 0) return;
+  int s1, s2;
   if (n & 1) {
+    ring_slots(h->cur, h->stepIdx, s1, s2);
+    if (!f.inj) h->cur = s2;
     h->stepIdx = 1 - h->stepIdx;
     h->wslot = 1 - h->wslot;
   }
   h->wvalid = true;
-  h->s1last = f.inj ? (h->cur + 1) % 3 : (h->cur + 2) % 3;   // the last step's stage-1 slot
+  // the last step's stage-1 slot: without sprays consecutive steps share it,
+  // with them it is the other parity's
+  ring_slots(h->cur, h->stepIdx, s1, s2);
+  h->s1last = f.inj ? s2 : s1;
   h->stepCount += n;
 }
 
@@ -871,7 +876,7 @@ int rn_batch_autotune(rn_batch b, int steps, int* chosen) {
   float bestMs = 1e30f;
   for (int shape = 0; shape < NTILES && e == cudaSuccess && rc == RN_OK; shape++) {
     if (rn_batch_set_tile(b, shape) != RN_OK) continue;    // a member's lists do not fit this shape
-    rc = rn_batch_step(b, PERIOD);                          // warm-up (builds the graph)
+    rc = rn_batch_step(b, GRAPH_STEPS);                     // warm-up (builds the graph)
     float ms = 0.0f;
     if (rc == RN_OK) e = cudaEventRecord(e0, b->stream);
     if (rc == RN_OK && e == cudaSuccess) rc = rn_batch_step(b, steps);

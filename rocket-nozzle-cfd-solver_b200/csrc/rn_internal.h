@@ -8,6 +8,29 @@
 #include "rn.h"
 #include "rn_kernels.cuh"
 
+// `steps` consecutive steps of a handle as a CUDA graph, and what they were
+// captured with (rn_step replays them only while all of that still holds).
+struct StepGraph {
+  cudaGraphExec_t exec = nullptr;
+  const void *K = nullptr, *base = nullptr, *xoff = nullptr;
+  int tile = -1, maxX = -1, nHeavy = -1;
+  int cur = -1, stepIdx = -1, wslot = -1, scur = -1;
+  int steps = 0;
+  long long launches = 0;
+  unsigned long long used = 0;
+  rn_params P = {};
+};
+
+// The state-ring slots of a step from slot cur: s1 takes the stage-1 state, s2
+// the step's result. The ring turns forwards and backwards in turn with the
+// step-info parity, so cur is back where it was, and the launches repeat,
+// every two steps.
+inline void ring_slots(int cur, int stepIdx, int& s1, int& s2) {
+  const int d = stepIdx ? 2 : 1;
+  s1 = (cur + d) % 3;
+  s2 = (cur + 2 * d) % 3;
+}
+
 // One solver instance: all of its device memory and its stream. The layout in
 // HBM is the reference's texture layout as plain arrays (see rn_api.cu).
 struct rn_solver {
@@ -76,16 +99,11 @@ struct rn_solver {
   int numSMs = 148;
   cudaStream_t side = nullptr;          // runs the heavy tiles' launch beside the main one
   cudaEvent_t evFork = nullptr, evJoin = nullptr;
-  // the 6-step period of non-spray steps as a CUDA graph, and what it was
-  // captured with (rn_step replays it only while all of that still holds)
-  cudaGraphExec_t stepGraph = nullptr;
-  const void* graphK = nullptr;
-  int graphTile = -1, graphMaxX = -1, graphHeavy = -1, graphCur = -1, graphStepIdx = -1, graphWslot = -1;
-  const void* graphBase = nullptr;
-  const void* graphXoff = nullptr;
-  rn_params graphP;
-  long long graphLaunches = 0;
-  int graphScur = -1, graphPeriod = 0;
+  // whole runs of steps as CUDA graphs, the least recently used one replaced
+  StepGraph graphs[2];
+  unsigned long long graphClock = 0;
+  int lastN = 0;             // the previous rn_step call's step count and parameters
+  rn_params lastP = {};
   unsigned* dHS = nullptr;   // the spray ring's (head, seed) on the device, for graph-replayed spray steps
   bool hsOnDevice = false;   // step_once launches read and advance dHS (while capturing)
   cudaStream_t sprayStream = nullptr;   // runs the parcel step beside stage 2 + the split step
@@ -112,6 +130,8 @@ struct rn_solver {
 
 // (Re)encode the tensor maps of h's state ring and pitched mask (rn_api.cu).
 int rn_build_tile_maps(rn_solver* h);
+// Destroy h's step graphs (their launches name its buffers and lists).
+void rn_drop_step_graphs(rn_solver* h);
 // Copy h->mask into its row-pitched copy (queued on h->stream).
 int rn_mask_refresh(rn_solver* h);
 // Record an error for rn_last_error() and return `code`.

@@ -104,7 +104,7 @@ struct ApplyArgs {
 // One instance of a batch: its buffers, where it stood in its state ring and
 // step-info ping-pong when the batch was (re)built, its first block in the
 // batch grid, and its parameter block. The kernels derive the slots of step k
-// from (cur0, stepIdx0, wslot0) and the step's BatchPhase.
+// from (cur0, stepIdx0, wslot0) and the step's BatchPhase (batch_ring).
 struct BatchInst {
   Grid g;
   float4* SA[3];
@@ -121,12 +121,22 @@ struct BatchInst {
   rn_params P;
 };
 struct BatchPhase {
-  int shift;                            // ring offset of this step: state slot s0 = (cur0 + shift) % 3
   int par;                              // step parity: stepIdx = stepIdx0 ^ par, wslot = wslot0 ^ par
+  int turn;                             // the ring has turned since parity 0 (not with sprays, whose steps end where they began)
   int finalCfl;                         // the launched kernel writes the step's final state
   int maxX;
   const int* active;                    // if set: per member, 0 = stopped (its blocks return at once)
 };
+
+// State-ring slots of member d in phase ph: s0 the step's base state, s1 its
+// stage-1 state, s2 its result. The ring turns by one slot pair forwards on even
+// step-info parity and back on odd (ring_slots in rn_internal.h).
+__host__ __device__ inline void batch_ring(const BatchInst& d, const BatchPhase& ph, int& s0, int& s1, int& s2) {
+  const int d0 = d.stepIdx0 ? 2 : 1, dk = (d.stepIdx0 ^ ph.par) ? 2 : 1;
+  s0 = (d.cur0 + (ph.turn ? 2 * d0 : 0)) % 3;
+  s1 = (s0 + dk) % 3;
+  s2 = (s0 + 2 * dk) % 3;
+}
 
 // The kernels are compiled twice from the same sources (rn_variant.cu):
 //   exact -- IEEE division and square root: every float operation rounds as

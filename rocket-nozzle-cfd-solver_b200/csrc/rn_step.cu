@@ -980,7 +980,8 @@ __device__ __forceinline__ void load_inst(const BatchInst* insts, int inst, Batc
 }
 // The step's stage arguments of instance d (stage 1 or 2 + the split step).
 __device__ __forceinline__ void batch_stage_args(const BatchInst& d, const BatchPhase& ph, int stage, StageArgs& a) {
-  const int s0 = (d.cur0 + ph.shift) % 3, s1 = (s0 + 1) % 3, s2 = (s0 + 2) % 3;
+  int s0, s1, s2;
+  batch_ring(d, ph, s0, s1, s2);
   const int si = d.stepIdx0 ^ ph.par, ws = d.wslot0 ^ ph.par;
   a.g = d.g;
   if (stage == 1) {
@@ -1033,7 +1034,8 @@ __global__ void __launch_bounds__(T::NT, T::MINB) k_stage2phys_batch(const Batch
   if (threadIdx.x == 0) {
     batch_stage_args(d, ph, 2, a);
     a.finalCfl = 0;
-    const int s0 = (d.cur0 + ph.shift) % 3, s1 = (s0 + 1) % 3, s2 = (s0 + 2) % 3;
+    int s0, s1, s2;
+    batch_ring(d, ph, s0, s1, s2);
     const int si = d.stepIdx0 ^ ph.par, ws = d.wslot0 ^ ph.par;
     p.g = d.g;
     p.A1 = d.SA[s1]; p.B1 = d.SB[s1]; p.A2 = d.SA[s2]; p.B2 = d.SB[s2]; p.oA = d.SA[s2]; p.oB = d.SB[s2];
