@@ -152,7 +152,7 @@ int alloc_buffers(rn_solver* h, int Nx, int Nr) {
   CK(cudaMemsetAsync(h->maskP, 0, size_t(h->maskPitch) * Nr, h->stream));
   CK(cudaMalloc(&h->errFlag, sizeof(unsigned)));
   CK(cudaMemsetAsync(h->errFlag, 0, sizeof(unsigned), h->stream));
-  CK(cudaMalloc(&h->dMaps, sizeof(TileMaps) * NTILES));
+  CK(cudaMalloc(&h->dMaps, sizeof(TileMaps) * NSHAPES));
   {
     const int rcm = rn_build_tile_maps(h);
     if (rcm != RN_OK) return rcm;
@@ -180,6 +180,7 @@ int alloc_buffers(rn_solver* h, int Nx, int Nr) {
   CK(cudaMalloc(&h->sortTemp, h->sortTempBytes > 0 ? h->sortTempBytes : 16));
   h->cur = 0; h->stepIdx = 0; h->wslot = 0; h->wvalid = false; h->stepCount = 0;
   h->seed = 1;
+  if (h->autoShape) h->shape = rn_auto_shape(Nx, Nr, h->numSMs);
   // empty topology (no groups) until a geometry is set
   h->hostMask.assign(N, 0);
   h->hostGeoM.assign(N * 4, 0.0f);
@@ -214,9 +215,9 @@ int rn_build_tile_maps(rn_solver* h) {
   const EncodeTiledFn enc = encode_tiled();
   if (!enc) return fail(RN_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the CUDA driver");
   const int Nx = h->Nx, Nr = h->Nr;
-  std::vector<TileMaps> maps(NTILES);
+  std::vector<TileMaps> maps(NSHAPES);
   const cuuint32_t estr[2] = {1, 1};
-  for (int t = 0; t < NTILES; t++) {
+  for (int t = 0; t < NSHAPES; t++) {
     const int PX = TILE_TX[t] + 4, PY = TILE_TY[t] + 4;
     const cuuint64_t pdim[2] = {cuuint64_t(4) * Nx, cuuint64_t(Nr)};
     const cuuint64_t pstride[1] = {cuuint64_t(16) * Nx};
@@ -248,7 +249,7 @@ int rn_build_tile_maps(rn_solver* h) {
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(RN_ERR_CUDA, "cuTensorMapEncodeTiled (geometry) failed: " + std::to_string(r));
   }
-  CK(cudaMemcpyAsync(h->dMaps, maps.data(), sizeof(TileMaps) * NTILES, cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemcpyAsync(h->dMaps, maps.data(), sizeof(TileMaps) * NSHAPES, cudaMemcpyHostToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   return RN_OK;
 }
@@ -259,12 +260,39 @@ int rn_mask_refresh(rn_solver* h) {
   return RN_OK;
 }
 
+static int rn_default_tile(int Nx, int Nr, int numSMs) {
+  return tile_count(RN_TILE_14x16, Nx, Nr) <= 3 * numSMs ? RN_TILE_14x16 : RN_TILE_16x15;
+}
+
+int rn_auto_shape(int Nx, int Nr, int numSMs) {
+  // All 10x10 blocks resident at once (3 an SM): a block's latency counts, not
+  // its share of halo work. 14x16 / 10x10, us per step: viscous 128x48 16.4 /
+  // 13.0, 256x96 17.5 / 15.2, 320x120 (384 blocks) 18.8 / 15.8; at 512x192 (3.5
+  // waves of 10x10 blocks) 21.9 / 33.
+  if (tile_count(SHAPE_SMALL, Nx, Nr) <= 3 * numSMs) return SHAPE_SMALL;
+  return rn_default_tile(Nx, Nr, numSMs);
+}
+
+int rn_use_shape(rn_solver* h, int shape) {
+  if (shape == h->shape) return RN_OK;
+  const int old = h->shape;
+  h->shape = shape;
+  const int rc = rn_build_member_lists(h);
+  if (rc != RN_OK) {
+    const std::string msg = g_err;
+    h->shape = old;
+    rn_build_member_lists(h);
+    return fail(rc, msg);
+  }
+  return RN_OK;
+}
+
 // Per tile, the cells outside it that belong to a cut-cell group with a cell
 // inside it (a sliver merged across the tile edge). Groups are a host plus the
 // slaves of its slave mask (geoM.z bits 1/2/4/8, cutcell.js:168-174).
 int rn_build_member_lists(rn_solver* h) {
   rn_drop_step_graphs(h);   // their launches name the old lists
-  const int TX = TILE_TX[h->tile], TY = TILE_TY[h->tile];
+  const int TX = TILE_TX[h->shape], TY = TILE_TY[h->shape];
   const int Nx = h->Nx, Nr = h->Nr, tx = (Nx + TX - 1) / TX, nT = tx * ((Nr + TY - 1) / TY);
   const uint8_t* mask = h->hostMask.data();
   const float* geoM = h->hostGeoM.data();
@@ -418,7 +446,7 @@ int rn_create(int Nx, int Nr, rn_handle* out) {
   }
   // default tile shape: 14x16 (compiled for 3 blocks per SM) when the grid's
   // tiles are all resident at 3 per SM at once, else 16x15
-  if (Nx > 0 && Nr > 0 && ((Nx + 13) / 14) * ((Nr + 15) / 16) <= 3 * h->numSMs) h->tile = RN_TILE_14x16;
+  if (Nx > 0 && Nr > 0) h->tile = rn_default_tile(Nx, Nr, h->numSMs);
   int rc = alloc_buffers(h, Nx, Nr);
   if (rc != RN_OK) {
     std::string msg = g_err;
@@ -588,9 +616,16 @@ int step_once(rn_solver* h, const rn_params* P) {
   a.finalCfl = 0;
   a.xoff = h->xoff; a.xcell = h->xcell; a.maxX = h->maxX;
   a.slotIn = s0; a.tm = h->dMaps; a.err = h->errFlag;
+  // The small shape's blocks leave room for the next kernel's, which set up
+  // (barrier, mask, geometry, member lists) while this one runs: 320x120 16.7 ->
+  // 15.8 us a viscous step, 12.3 -> 11.3 an inviscid one. Not for the larger
+  // shapes: as slots come free one by one, consecutive blocks, the costly ones
+  // of a wall among them, gather on one SM (14x16, viscous 512x192: 21.9 ->
+  // 23.2 us).
+  a.pdl = !inj && !h->prof && h->shape == SHAPE_SMALL;
   {
     ProfScope ps(h, RN_K_STAGE1);
-    h->K->stage1(a, *P, h->tile, h->stream);
+    h->K->stage1(a, *P, h->shape, h->stream);
   }
   h->launches++;
   if (inj) {
@@ -656,17 +691,17 @@ int step_once(rn_solver* h, const rn_params* P) {
       }
       CK(cudaEventRecord(h->evFork, h->stream));
       CK(cudaStreamWaitEvent(h->side, h->evFork, 0));
-      h->K->stage2phys(b, p, *P, h->tile, h->heavy, h->nHeavy, false, h->side);
+      h->K->stage2phys(b, p, *P, h->shape, h->heavy, h->nHeavy, false, h->side);
       CK(cudaEventRecord(h->evJoin, h->side));
-      h->K->stage2phys(b, p, *P, h->tile, nullptr, h->nHeavy, true, h->stream);
+      h->K->stage2phys(b, p, *P, h->shape, nullptr, h->nHeavy, true, h->stream);
       CK(cudaStreamWaitEvent(h->stream, h->evJoin, 0));
       h->launches++;
     } else {
-      h->K->stage2phys(b, p, *P, h->tile, nullptr, 0, false, h->stream);
+      h->K->stage2phys(b, p, *P, h->shape, nullptr, 0, false, h->stream);
     }
   } else {
     ProfScope ps(h, RN_K_STAGE2);
-    h->K->stage2(b, *P, h->tile, h->stream);
+    h->K->stage2(b, *P, h->shape, h->stream);
   }
   h->launches++;
   h->cur = s2;
@@ -704,7 +739,7 @@ int step_once(rn_solver* h, const rn_params* P) {
 // kernels, launch shapes, buffers and parameter block that hold now, from the
 // ring position the handle is at (up to one step of the two-step period).
 bool graph_matches(const rn_solver* h, const StepGraph& g, const rn_params* P) {
-  return g.exec && g.K == h->K && g.tile == h->tile && g.maxX == h->maxX && g.nHeavy == h->nHeavy &&
+  return g.exec && g.K == h->K && g.tile == h->shape && g.maxX == h->maxX && g.nHeavy == h->nHeavy &&
          g.base == h->SA[0] && g.xoff == h->xoff && std::memcmp(&g.P, P, sizeof(rn_params)) == 0;
 }
 bool graph_at_start(const rn_solver* h, const StepGraph& g, bool inj) {
@@ -772,7 +807,7 @@ int capture_steps(rn_solver* h, const rn_params* P, int B, StepGraph& g) {
   if (gr) cudaGraphDestroy(gr);
   if (rc != RN_OK) return rc;
   g.K = h->K; g.base = h->SA[0]; g.xoff = h->xoff;
-  g.tile = h->tile; g.maxX = h->maxX; g.nHeavy = h->nHeavy;
+  g.tile = h->shape; g.maxX = h->maxX; g.nHeavy = h->nHeavy;
   g.cur = cur; g.stepIdx = stepIdx; g.wslot = wslot; g.scur = scur;
   g.steps = B;
   g.P = *P;
@@ -1212,16 +1247,10 @@ int rn_set_precision(rn_handle h, int mode) {
 int rn_set_tile(rn_handle h, int shape) {
   if (!valid(h) || shape < 0 || shape >= NTILES) return fail(RN_ERR_ARG, "rn_set_tile: bad handle or shape");
   if (h->batch) return fail(RN_ERR_STATE, "rn_set_tile: the handle is in a batch");
-  if (shape == h->tile) return RN_OK;
-  const int old = h->tile;
+  const int rc = rn_use_shape(h, shape);
+  if (rc != RN_OK) return rc;
   h->tile = shape;
-  int rc = rn_build_member_lists(h);
-  if (rc != RN_OK) {
-    std::string msg = g_err;
-    h->tile = old;
-    rn_build_member_lists(h);
-    return fail(rc, msg);
-  }
+  h->autoShape = false;
   return RN_OK;
 }
 
@@ -1267,13 +1296,17 @@ int rn_autotune(rn_handle h, const rn_params* P, int steps, int* chosen) {
   const int prof = h->prof;
   h->prof = 0;
   cudaError_t e = copy_all(true);
-  int best = h->tile, rc = RN_OK;
+  // the public shapes, then the one an unset handle of this grid runs
+  const int unset = rn_auto_shape(h->Nx, h->Nr, h->numSMs);
+  int best = h->shape, rc = RN_OK;
   float bestMs = 1e30f;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (e == cudaSuccess) e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
-  for (int shape = 0; shape < NTILES && e == cudaSuccess && rc == RN_OK; shape++) {
-    h->tile = shape;
+  for (int q = 0; q <= NTILES && e == cudaSuccess && rc == RN_OK; q++) {
+    const int shape = q < NTILES ? q : unset;
+    if (q == NTILES && unset < NTILES) break;
+    h->shape = shape;
     rc = rn_build_member_lists(h);
     if (rc != RN_OK) { rc = RN_OK; continue; }          // this shape cannot hold the geometry's lists
     rc = rn_step(h, 2, P);                                // warm-up
@@ -1298,12 +1331,14 @@ int rn_autotune(rn_handle h, const rn_params* P, int steps, int* chosen) {
   cudaFree(save);
   h->launches = launches;
   h->prof = prof;
-  h->tile = best;
+  h->shape = best;
+  h->autoShape = best >= NTILES;
+  h->tile = best < NTILES ? best : rn_default_tile(h->Nx, h->Nr, h->numSMs);
   int rc2 = rn_build_member_lists(h);
   if (e != cudaSuccess) return cuda_fail(e, "rn_autotune");
   if (rc != RN_OK) return rc;
   if (rc2 != RN_OK) return rc2;
-  if (chosen) *chosen = best;
+  if (chosen) *chosen = h->tile;
   return RN_OK;
 }
 

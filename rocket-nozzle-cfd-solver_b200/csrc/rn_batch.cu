@@ -489,7 +489,7 @@ int prepare(rn_batch_t* b) {
   const KernelSet* K = b->members[0]->K;
   for (rn_solver* h : b->members) {
     if (h->K != K) return bfail(RN_ERR_STATE, "rn_batch_step: members have different precisions");
-    if (h->tile != b->tile) return bfail(RN_ERR_STATE, "rn_batch_step: a member's tile shape differs from the batch's");
+    if (h->shape != b->tile) return bfail(RN_ERR_STATE, "rn_batch_step: a member's tile shape differs from the batch's");
     if (!h->SA[0]) return bfail(RN_ERR_STATE, "rn_batch_step: a member has no buffers");
   }
   b->K = K;
@@ -730,7 +730,7 @@ int rn_batch_add(rn_batch b, rn_handle h, const rn_params* P, int* slot) {
     if (!(f == b->flags)) return bfail(RN_ERR_ARG, "rn_batch_add: physics flags (visc, chem, inj) differ from the batch's");
     if (h->K != b->members[0]->K) return bfail(RN_ERR_ARG, "rn_batch_add: precision differs from the batch's");
   }
-  if (h->tile != b->tile) {
+  if (h->tile != b->tile || h->shape != b->tile) {
     int rc = rn_set_tile(h, b->tile);
     if (rc != RN_OK) return rc;
   }

@@ -88,7 +88,10 @@ struct rn_solver {
   long long profN[RN_NKERNELS] = {0};
   // tile shape of the stage/physics kernels and, per tile, the out-of-tile
   // members of its cut-cell groups (built from host copies of the topology)
-  int tile = RN_TILE_16x15;
+  // (tile: the public name; shape: what its kernels run, TILE_TX/TILE_TY's index.
+  // They differ only while autoShape, i.e. until a caller sets the tile shape)
+  int tile = RN_TILE_16x15, shape = RN_TILE_16x15;
+  bool autoShape = true;
   int* xoff = nullptr;
   int* xcell = nullptr;
   int maxX = 1;
@@ -137,6 +140,10 @@ int rn_mask_refresh(rn_solver* h);
 // Record an error for rn_last_error() and return `code`.
 int rn_record_error(int code, const std::string& msg);
 int rn_record_cuda(cudaError_t e, const char* what);
+// The shape a handle with an Nx x Nr grid runs when no caller set one.
+int rn_auto_shape(int Nx, int Nr, int numSMs);
+// Makes `shape` the one that h's kernels run and rebuilds its member lists.
+int rn_use_shape(rn_solver* h, int shape);
 // (Re)build the per-tile member lists of `h` for its current tile shape.
 int rn_build_member_lists(rn_solver* h);
 // Make h->wmax[h->wslot] the wave-speed max of the current state if it is not.

@@ -21,11 +21,20 @@ namespace rn {
 // 14x16 spreads a 512x192 grid over 37 x 12 = 444 tiles, 3 per SM on 148 SMs,
 // and is compiled for those 3 blocks (24 warps: 80 registers, no spills); the
 // others for 32 resident warps (64 registers).
-constexpr int NTILES = 5;
-constexpr int TILE_TX[NTILES] = {16, 16, 16, 32, 14};
-constexpr int TILE_TY[NTILES] = {16, 8, 15, 15, 16};
-constexpr int TILE_NT[NTILES] = {256, 128, 256, 512, 256};
-constexpr int TILE_WARPS[NTILES] = {32, 32, 32, 32, 24};
+// The last shape has no public name: a handle whose tile shape nobody set runs
+// it on small grids (auto_shape). 10x10 cells on 256 threads fill each phase in
+// one pass (196 primitives, 220 faces, 100 updates beside 144 vcell slots),
+// where 14x16 takes two: with one or two blocks an SM a block's latency is the
+// kernel's time.
+constexpr int NTILES = 5, NSHAPES = 6;   // public shapes (RN_TILE_*), all compiled shapes
+constexpr int TILE_TX[NSHAPES] = {16, 16, 16, 32, 14, 10};
+constexpr int TILE_TY[NSHAPES] = {16, 8, 15, 15, 16, 10};
+constexpr int TILE_NT[NSHAPES] = {256, 128, 256, 512, 256, 256};
+constexpr int TILE_WARPS[NSHAPES] = {32, 32, 32, 32, 24, 24};
+constexpr int SHAPE_SMALL = 5;
+inline int tile_count(int shape, int Nx, int Nr) {
+  return ((Nx + TILE_TX[shape] - 1) / TILE_TX[shape]) * ((Nr + TILE_TY[shape] - 1) / TILE_TY[shape]);
+}
 // Most out-of-tile group members one tile may list (set_geometry rejects more).
 constexpr int MAXX = 64;
 // Tiles listing more out-of-tile members than this run the fused stage-2 +
@@ -56,6 +65,7 @@ struct StageArgs {
   int slotIn;                           // ring slot of (A, B): selects the tensor maps of the halo copy
   const TileMaps* tm;                   // the handle's tensor maps, one TileMaps per tile shape
   unsigned* err;                        // set when a halo copy did not complete in time
+  int pdl;                              // launch with programmatic dependence on the kernel before it
 };
 
 struct PhysArgs {

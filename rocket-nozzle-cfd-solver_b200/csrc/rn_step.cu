@@ -57,6 +57,8 @@ struct TileT {
   // memory, loop body and live registers cost more than they save (64 batched
   // instances, 16x15: 4.37 -> 4.18 G).
   static constexpr bool WIDE = WARPS_ < 32;
+  // launched with programmatic dependence on the kernel before it (rn_api.cu)
+  static constexpr bool PDL = ID_ == SHAPE_SMALL;
   static constexpr int PX = TX + 4, PY = TY + 4, NPT = PX * PY;   // primitives with a 2-cell halo
   static constexpr int NXF = TY * (TX + 1), NRF = (TY + 1) * TX;  // x- and r-faces of a tile
   static constexpr int TW = TX + 2, NTT = (TX + 2) * (TY + 2);    // vcell ring (tile + 1)
@@ -80,8 +82,9 @@ using Tile1 = TileT<TILE_TX[1], TILE_TY[1], TILE_NT[1], TILE_WARPS[1], 1>;
 using Tile2 = TileT<TILE_TX[2], TILE_TY[2], TILE_NT[2], TILE_WARPS[2], 2>;
 using Tile3 = TileT<TILE_TX[3], TILE_TY[3], TILE_NT[3], TILE_WARPS[3], 3>;
 using Tile4 = TileT<TILE_TX[4], TILE_TY[4], TILE_NT[4], TILE_WARPS[4], 4>;
+using Tile5 = TileT<TILE_TX[5], TILE_TY[5], TILE_NT[5], TILE_WARPS[5], 5>;
 static_assert(Tile0::NC <= Tile0::NT && Tile1::NC <= Tile1::NT && Tile2::NC <= Tile2::NT && Tile3::NC <= Tile3::NT &&
-                  Tile4::NC <= Tile4::NT,
+                  Tile4::NC <= Tile4::NT && Tile5::NC <= Tile5::NT,
               "a thread per cell");
 static_assert(4 * Tile3::PX <= 256 && Tile3::MW <= 256 && Tile0::PY <= 256, "copy boxes within 256 elements");
 
@@ -202,22 +205,34 @@ __device__ __forceinline__ float member_face_area(const Grid& g, int q, const in
 }
 
 // Start of a stage kernel's block: thread 0 initialises the halo copy's
-// mbarrier and issues the three tiled copies of the tile + 2-cell halo (raw A
-// into R, raw B into R + NPT8, the mask block into sMask). The mask box starts
-// at the 16-byte boundary at or below the halo's first column.
+// mbarrier and issues its tiled copies: the state of the tile + 2-cell halo
+// (raw A into R, raw B into R + NPT8), the mask block (its box starts at the
+// 16-byte boundary at or below the halo's first column) and, for WIDE shapes,
+// the geometry boxes. With dependent launches (PDL) the mask and geometry,
+// which no kernel of the step writes, go first, then, after the kernel before,
+// the state it wrote. The other threads meanwhile load face areas and the
+// member list.
 template <class T>
 __device__ __forceinline__ void halo_issue(const TileMaps* tm, int slot, int x0, int y0, float4* R, uint8_t* sMask,
                                            uint64_t* bar) {
+  if constexpr (T::PDL) pdl_launch();
   if (threadIdx.x == 0) {
     const TileMaps& M = tm[T::ID];
     mbar_init(bar, 1);
     mbar_expect_tx(bar, T::HALO_BYTES + (T::WIDE ? T::GEO_BYTES : 0u));
-    tma_load_2d(R, &M.a[slot], 4 * (x0 - 2), y0 - 2, bar);
-    tma_load_2d(R + T::NPT8, &M.b[slot], 4 * (x0 - 2), y0 - 2, bar);
+    if constexpr (!T::PDL) {
+      tma_load_2d(R, &M.a[slot], 4 * (x0 - 2), y0 - 2, bar);
+      tma_load_2d(R + T::NPT8, &M.b[slot], 4 * (x0 - 2), y0 - 2, bar);
+    }
     tma_load_2d(sMask, &M.mask, (x0 - 2) & ~15, y0 - 2, bar);
     if constexpr (T::WIDE) {                     // geoM ring box, then geoG tile box, after the raw block
       tma_load_2d(R + 2 * T::NPT8, &M.geoM, 4 * (x0 - 1), y0 - 1, bar);
       tma_load_2d(R + 2 * T::NPT8 + T::NGM8, &M.geoG, 4 * x0, y0, bar);
+    }
+    if constexpr (T::PDL) {
+      pdl_wait();
+      tma_load_2d(R, &M.a[slot], 4 * (x0 - 2), y0 - 2, bar);
+      tma_load_2d(R + T::NPT8, &M.b[slot], 4 * (x0 - 2), y0 - 2, bar);
     }
   }
 }
@@ -549,8 +564,11 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
   float* sAr = reinterpret_cast<float*>(R + stage_region_t<T>(xn));
   float4* sW = reinterpret_cast<float4*>(sAr) + (NF + 3) / 4;
   float4* sWb = sW + NP;
-  for (int q = tid; q < xn; q += NT) xc[q] = a.xcell[xb + q];
+  // (by the last threads: the first may wait for the kernel before)
+  for (int q = NT - 1 - tid; q < xn; q += NT) xc[q] = a.xcell[xb + q];
 
+  // from here on the block reads and writes what the kernel before it wrote or read
+  if constexpr (T::PDL) pdl_wait();
   float dt, t;
   if (STAGE == 1) {
     float4 prev = *a.stPrev;
@@ -847,7 +865,8 @@ __device__ __forceinline__ void stage2_physics_body(const StageArgs& a, const Ph
   float* sAr = reinterpret_cast<float*>(sB2 + T::NC + xn);   // face areas, kept for FS_SOURCE
   float4* sW = reinterpret_cast<float4*>(sAr) + (NF + 3) / 4;
   float4* sWb = sW + NP;
-  for (int q = tid; q < xn; q += NT) xc[q] = a.xcell[xb + q];
+  for (int q = NT - 1 - tid; q < xn; q += NT) xc[q] = a.xcell[xb + q];
+  if constexpr (T::PDL) pdl_wait();
   const float4 st = *a.stNew;
   const float dt = st.x, t = st.z;
   __syncthreads();
@@ -1200,57 +1219,79 @@ static int init_tile() {
 // what a member list of MAXX cells needs (process-wide function attributes).
 int stage_kernels_init() {
   return (init_tile<Tile0>() == 0 && init_tile<Tile1>() == 0 && init_tile<Tile2>() == 0 && init_tile<Tile3>() == 0 &&
-          init_tile<Tile4>() == 0)
+          init_tile<Tile4>() == 0 && init_tile<Tile5>() == 0)
              ? 0
              : -1;
 }
 
-void launch_stage1(const StageArgs& a, const rn_params& P, int tile, cudaStream_t s) {
-  if (tile == 4) k_stage<Tile4, 1><<<tiles_of<Tile4>(a.g), Tile4::NT, stage_smem_t<Tile4>(a.maxX), s>>>(a, P);
-  else if (tile == 3) k_stage<Tile3, 1><<<tiles_of<Tile3>(a.g), Tile3::NT, stage_smem_t<Tile3>(a.maxX), s>>>(a, P);
-  else if (tile == 2) k_stage<Tile2, 1><<<tiles_of<Tile2>(a.g), Tile2::NT, stage_smem_t<Tile2>(a.maxX), s>>>(a, P);
-  else if (tile == 1) k_stage<Tile1, 1><<<tiles_of<Tile1>(a.g), Tile1::NT, stage_smem_t<Tile1>(a.maxX), s>>>(a, P);
-  else k_stage<Tile0, 1><<<tiles_of<Tile0>(a.g), Tile0::NT, stage_smem_t<Tile0>(a.maxX), s>>>(a, P);
+// A launch that may start its blocks before the kernel ahead of it in the
+// stream has completed (`pdl`; the kernel then waits for it itself).
+template <class... A, class... B>
+static void launch_step(void (*kernel)(A...), dim3 grid, int threads, size_t smem, cudaStream_t s, bool pdl,
+                        const B&... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, args...);
 }
-void launch_stage2(const StageArgs& a, const rn_params& P, int tile, cudaStream_t s) {
-  if (tile == 4) k_stage<Tile4, 2><<<tiles_of<Tile4>(a.g), Tile4::NT, stage_smem_t<Tile4>(a.maxX), s>>>(a, P);
-  else if (tile == 3) k_stage<Tile3, 2><<<tiles_of<Tile3>(a.g), Tile3::NT, stage_smem_t<Tile3>(a.maxX), s>>>(a, P);
-  else if (tile == 2) k_stage<Tile2, 2><<<tiles_of<Tile2>(a.g), Tile2::NT, stage_smem_t<Tile2>(a.maxX), s>>>(a, P);
-  else if (tile == 1) k_stage<Tile1, 2><<<tiles_of<Tile1>(a.g), Tile1::NT, stage_smem_t<Tile1>(a.maxX), s>>>(a, P);
-  else k_stage<Tile0, 2><<<tiles_of<Tile0>(a.g), Tile0::NT, stage_smem_t<Tile0>(a.maxX), s>>>(a, P);
+template <class T, int STAGE>
+static void stage_t(const StageArgs& a, const rn_params& P, cudaStream_t s) {
+  launch_step(k_stage<T, STAGE>, tiles_of<T>(a.g), T::NT, stage_smem_t<T>(a.maxX), s, a.pdl != 0, a, P);
 }
+template <int STAGE>
+static void launch_stage(const StageArgs& a, const rn_params& P, int tile, cudaStream_t s) {
+  if (tile == 5) stage_t<Tile5, STAGE>(a, P, s);
+  else if (tile == 4) stage_t<Tile4, STAGE>(a, P, s);
+  else if (tile == 3) stage_t<Tile3, STAGE>(a, P, s);
+  else if (tile == 2) stage_t<Tile2, STAGE>(a, P, s);
+  else if (tile == 1) stage_t<Tile1, STAGE>(a, P, s);
+  else stage_t<Tile0, STAGE>(a, P, s);
+}
+void launch_stage1(const StageArgs& a, const rn_params& P, int tile, cudaStream_t s) { launch_stage<1>(a, P, tile, s); }
+void launch_stage2(const StageArgs& a, const rn_params& P, int tile, cudaStream_t s) { launch_stage<2>(a, P, tile, s); }
 // heavy != nullptr: the heavy tiles alone (nHeavy blocks, shared memory for
 // their lists); otherwise every tile, with the heavy ones skipped when `skip`
 // (they then run in the other launch, on another stream at the same time).
 template <class T>
 static void stage2phys_t(const StageArgs& a, const PhysArgs& p, const rn_params& P, const int* heavy, int nHeavy,
                          bool skip, cudaStream_t s) {
+  const int* none = nullptr;
   if (heavy) {
-    k_stage2phys<T><<<nHeavy, T::NT, fused_smem_t<T>(a.maxX), s>>>(a, p, P, heavy, -1);
+    launch_step(k_stage2phys<T>, dim3(nHeavy), T::NT, fused_smem_t<T>(a.maxX), s, false, a, p, P, heavy, -1);
   } else if (skip) {
     const int xs = a.maxX < XSMALL ? a.maxX : XSMALL;
-    k_stage2phys<T><<<tiles_of<T>(a.g), T::NT, fused_smem_t<T>(xs), s>>>(a, p, P, nullptr, XSMALL);
+    launch_step(k_stage2phys<T>, tiles_of<T>(a.g), T::NT, fused_smem_t<T>(xs), s, false, a, p, P, none, XSMALL);
   } else {
-    k_stage2phys<T><<<tiles_of<T>(a.g), T::NT, fused_smem_t<T>(a.maxX), s>>>(a, p, P, nullptr, -1);
+    launch_step(k_stage2phys<T>, tiles_of<T>(a.g), T::NT, fused_smem_t<T>(a.maxX), s, a.pdl != 0, a, p, P, none, -1);
   }
 }
 void launch_stage2phys(const StageArgs& a, const PhysArgs& p, const rn_params& P, int tile, const int* heavy,
                        int nHeavy, bool skip, cudaStream_t s) {
-  if (tile == 4) stage2phys_t<Tile4>(a, p, P, heavy, nHeavy, skip, s);
+  if (tile == 5) stage2phys_t<Tile5>(a, p, P, heavy, nHeavy, skip, s);
+  else if (tile == 4) stage2phys_t<Tile4>(a, p, P, heavy, nHeavy, skip, s);
   else if (tile == 3) stage2phys_t<Tile3>(a, p, P, heavy, nHeavy, skip, s);
   else if (tile == 2) stage2phys_t<Tile2>(a, p, P, heavy, nHeavy, skip, s);
   else if (tile == 1) stage2phys_t<Tile1>(a, p, P, heavy, nHeavy, skip, s);
   else stage2phys_t<Tile0>(a, p, P, heavy, nHeavy, skip, s);
 }
 void launch_batch_stage1(const BatchInst* d, const int* bi, int nb, BatchPhase ph, int tile, cudaStream_t s) {
-  if (tile == 4) k_stage_batch<Tile4, 1><<<nb, Tile4::NT, stage_smem_t<Tile4>(ph.maxX), s>>>(d, bi, ph);
+  if (tile == 5) k_stage_batch<Tile5, 1><<<nb, Tile5::NT, stage_smem_t<Tile5>(ph.maxX), s>>>(d, bi, ph);
+  else if (tile == 4) k_stage_batch<Tile4, 1><<<nb, Tile4::NT, stage_smem_t<Tile4>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 3) k_stage_batch<Tile3, 1><<<nb, Tile3::NT, stage_smem_t<Tile3>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 2) k_stage_batch<Tile2, 1><<<nb, Tile2::NT, stage_smem_t<Tile2>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 1) k_stage_batch<Tile1, 1><<<nb, Tile1::NT, stage_smem_t<Tile1>(ph.maxX), s>>>(d, bi, ph);
   else k_stage_batch<Tile0, 1><<<nb, Tile0::NT, stage_smem_t<Tile0>(ph.maxX), s>>>(d, bi, ph);
 }
 void launch_batch_stage2(const BatchInst* d, const int* bi, int nb, BatchPhase ph, int tile, cudaStream_t s) {
-  if (tile == 4) k_stage_batch<Tile4, 2><<<nb, Tile4::NT, stage_smem_t<Tile4>(ph.maxX), s>>>(d, bi, ph);
+  if (tile == 5) k_stage_batch<Tile5, 2><<<nb, Tile5::NT, stage_smem_t<Tile5>(ph.maxX), s>>>(d, bi, ph);
+  else if (tile == 4) k_stage_batch<Tile4, 2><<<nb, Tile4::NT, stage_smem_t<Tile4>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 3) k_stage_batch<Tile3, 2><<<nb, Tile3::NT, stage_smem_t<Tile3>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 2) k_stage_batch<Tile2, 2><<<nb, Tile2::NT, stage_smem_t<Tile2>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 1) k_stage_batch<Tile1, 2><<<nb, Tile1::NT, stage_smem_t<Tile1>(ph.maxX), s>>>(d, bi, ph);
@@ -1271,7 +1312,8 @@ static void batch_stage2phys_t(const BatchInst* d, const int* bi, int nb, BatchP
 }
 void launch_batch_stage2phys(const BatchInst* d, const int* bi, int nb, BatchPhase ph, int tile, const int2* heavy,
                              int nHeavy, bool skip, cudaStream_t s) {
-  if (tile == 4) batch_stage2phys_t<Tile4>(d, bi, nb, ph, heavy, nHeavy, skip, s);
+  if (tile == 5) batch_stage2phys_t<Tile5>(d, bi, nb, ph, heavy, nHeavy, skip, s);
+  else if (tile == 4) batch_stage2phys_t<Tile4>(d, bi, nb, ph, heavy, nHeavy, skip, s);
   else if (tile == 3) batch_stage2phys_t<Tile3>(d, bi, nb, ph, heavy, nHeavy, skip, s);
   else if (tile == 2) batch_stage2phys_t<Tile2>(d, bi, nb, ph, heavy, nHeavy, skip, s);
   else if (tile == 1) batch_stage2phys_t<Tile1>(d, bi, nb, ph, heavy, nHeavy, skip, s);

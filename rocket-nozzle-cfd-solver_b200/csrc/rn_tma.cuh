@@ -32,6 +32,11 @@ struct TileMaps {
 __host__ __device__ constexpr int mask_box_width(int PX) { return ((PX + 15 + 15) / 16) * 16; }
 
 #ifdef __CUDACC__
+// Programmatic dependent launch: wait until the kernel before this one in the
+// stream has completed and its writes are visible; let the next one start its
+// blocks (which wait the same way). Both do nothing in an ordinary launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
   return static_cast<unsigned>(__cvta_generic_to_shared(p));
 }
