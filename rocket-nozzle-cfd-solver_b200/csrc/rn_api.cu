@@ -270,7 +270,11 @@ int rn_auto_shape(int Nx, int Nr, int numSMs) {
   // 13.0, 256x96 17.5 / 15.2, 320x120 (384 blocks) 18.8 / 15.8; at 512x192 (3.5
   // waves of 10x10 blocks) 21.9 / 33.
   if (tile_count(SHAPE_SMALL, Nx, Nr) <= 3 * numSMs) return SHAPE_SMALL;
-  return rn_default_tile(Nx, Nr, numSMs);
+  const int tile = rn_default_tile(Nx, Nr, numSMs);
+  if (tile == RN_TILE_16x15 &&
+      prefer_16x16(tile_count(RN_TILE_16x16, Nx, Nr), tile_count(RN_TILE_16x15, Nx, Nr)))
+    return RN_TILE_16x16;
+  return tile;
 }
 
 int rn_use_shape(rn_solver* h, int shape) {
@@ -537,9 +541,17 @@ int rn_set_geometry(rn_handle h, const uint8_t* mask, const float* geoA, const f
   h->hostMask.resize(N);
   for (size_t k = 0; k < N; k++) h->hostMask[k] = mask[k] ? 1 : 0;
   h->hostGeoM.assign(geoM, geoM + 4 * N);
+  const int oldShape = h->shape;
+  if (h->autoShape) h->shape = rn_auto_shape(Nx, Nr, h->numSMs);
   int rc = rn_build_member_lists(h);
+  if (h->autoShape && h->shape == RN_TILE_16x16 && (rc != RN_OK || h->maxX > XSMALL)) {
+    // long lists cost 16x16 blocks their fourth place on an SM
+    h->shape = RN_TILE_16x15;
+    rc = rn_build_member_lists(h);
+  }
   if (rc != RN_OK) {
     std::string msg = g_err;
+    h->shape = oldShape;
     h->hostMask = std::move(oldMask);
     h->hostGeoM = std::move(oldGeoM);
     rn_build_member_lists(h);

@@ -48,7 +48,9 @@ struct rn_batch_t {
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;           // end of the last rn_batch_step
   cudaEvent_t staged = nullptr;         // the last descriptor upload has read the pinned buffer
-  int tile = RN_TILE_16x15;
+  int tile = RN_TILE_16x15;             // public name
+  int shape = RN_TILE_16x15;            // what the kernels run; not `tile` only while autoShape
+  bool autoShape = true;                // nobody set the tile shape
   Flags flags;
   std::vector<rn_solver*> members;
   std::vector<rn_params> params;
@@ -129,7 +131,7 @@ void normalise(const rn_batch_t* b, const rn_solver* h, int& cur0, int& si0, int
 // member lists up to date with the handles.
 int refresh(rn_batch_t* b) {
   const int nm = int(b->members.size());
-  const int TX = TILE_TX[b->tile], TY = TILE_TY[b->tile];
+  const int TX = TILE_TX[b->shape], TY = TILE_TY[b->shape];
   // block table: rebuilt when a member's grid size changed
   // (members stopped in a run have no blocks: grid size 0 x 0 in the table)
   std::vector<int> layout(2 * nm);
@@ -253,7 +255,7 @@ int launch_step(rn_batch_t* b, int c, bool withSpray) {
   ph.active = b->runActive.empty() ? nullptr : b->dActive;
   const int nb = b->nblocks;
   ph.finalCfl = 0;
-  b->K->batchStage1(b->dInst, b->dBlock, nb, ph, b->tile, b->stream);
+  b->K->batchStage1(b->dInst, b->dBlock, nb, ph, b->shape, b->stream);
   b->launches++;
   if (f.inj && withSpray) {
     // GPUSpray.step between the two stages (solver.js:865-871), per member, on
@@ -302,16 +304,16 @@ int launch_step(rn_batch_t* b, int c, bool withSpray) {
       // the few tiles with long member lists on the side stream, at the same time
       cudaEventRecord(b->evFork, b->stream);
       cudaStreamWaitEvent(b->side, b->evFork, 0);
-      b->K->batchStage2Phys(b->dInst, b->dBlock, nb, ph, b->tile, b->dHeavy, b->nHeavy, false, b->side);
+      b->K->batchStage2Phys(b->dInst, b->dBlock, nb, ph, b->shape, b->dHeavy, b->nHeavy, false, b->side);
       cudaEventRecord(b->evJoin, b->side);
-      b->K->batchStage2Phys(b->dInst, b->dBlock, nb, ph, b->tile, nullptr, b->nHeavy, true, b->stream);
+      b->K->batchStage2Phys(b->dInst, b->dBlock, nb, ph, b->shape, nullptr, b->nHeavy, true, b->stream);
       cudaStreamWaitEvent(b->stream, b->evJoin, 0);
       b->launches++;
     } else {
-      b->K->batchStage2Phys(b->dInst, b->dBlock, nb, ph, b->tile, nullptr, 0, false, b->stream);
+      b->K->batchStage2Phys(b->dInst, b->dBlock, nb, ph, b->shape, nullptr, 0, false, b->stream);
     }
   } else {
-    b->K->batchStage2(b->dInst, b->dBlock, nb, ph, b->tile, b->stream);
+    b->K->batchStage2(b->dInst, b->dBlock, nb, ph, b->shape, b->stream);
   }
   b->launches++;
   if (f.inj && withSpray) {
@@ -366,7 +368,7 @@ int build_graph(rn_batch_t* b) {
   }
   b->graphK = b->K;
   b->graphBlocks = b->nblocks;
-  b->graphTile = b->tile;
+  b->graphTile = b->shape;
   b->graphMaxX = b->maxX;
   b->graphHeavy = b->split ? b->nHeavy : 0;
   b->graphFlags = b->flags;
@@ -398,7 +400,7 @@ int issue_steps(rn_batch_t* b, int n) {
   }
   if (n - done >= GRAPH_STEPS) {
     const int* active = b->runActive.empty() ? nullptr : b->dActive;
-    if (!b->graph || b->graphK != b->K || b->graphBlocks != b->nblocks || b->graphTile != b->tile ||
+    if (!b->graph || b->graphK != b->K || b->graphBlocks != b->nblocks || b->graphTile != b->shape ||
         b->graphMaxX != b->maxX || b->graphHeavy != (b->split ? b->nHeavy : 0) || !(b->graphFlags == b->flags) ||
         b->graphActive != active) {
       rc = build_graph(b);
@@ -483,13 +485,48 @@ int run_buffers(rn_batch_t* b, size_t nm) {
   return RN_OK;
 }
 
+// Makes `shape` the one the batch and its members run.
+int use_shape(rn_batch_t* b, int shape) {
+  if (shape == b->shape) return RN_OK;
+  BCK(cudaStreamSynchronize(b->stream));
+  for (size_t m = 0; m < b->members.size(); m++) {
+    const int rc = rn_use_shape(b->members[m], shape);
+    if (rc != RN_OK) {
+      const std::string msg = rn_last_error();
+      for (size_t q = 0; q < m; q++) rn_use_shape(b->members[q], b->shape);
+      return bfail(rc, msg);
+    }
+  }
+  b->shape = shape;
+  b->layout.clear();   // block table and descriptors are rebuilt by the next step
+  b->uploaded.clear();
+  return RN_OK;
+}
+
+// Brings h, about to join, and the batch to one shape: the one set, or, while
+// nobody set one, the one that suits the members' grids and h's.
+int join_shape(rn_batch_t* b, rn_solver* h) {
+  if (b->autoShape) {
+    long long t16 = tile_count(RN_TILE_16x16, h->Nx, h->Nr), t15 = tile_count(RN_TILE_16x15, h->Nx, h->Nr);
+    for (const rn_solver* q : b->members) {
+      t16 += tile_count(RN_TILE_16x16, q->Nx, q->Nr);
+      t15 += tile_count(RN_TILE_16x15, q->Nx, q->Nr);
+    }
+    if (prefer_16x16(t16, t15) && use_shape(b, RN_TILE_16x16) == RN_OK && rn_use_shape(h, RN_TILE_16x16) == RN_OK)
+      return RN_OK;
+    const int rc = use_shape(b, RN_TILE_16x15);   // (or 16x16's lists are too long)
+    if (rc != RN_OK) return rc;
+  }
+  return rn_use_shape(h, b->shape);
+}
+
 // Checks the batch's members before a step (rn_batch_step, rn_batch_run) and
 // orders their queued work before the batch's kernels.
 int prepare(rn_batch_t* b) {
   const KernelSet* K = b->members[0]->K;
   for (rn_solver* h : b->members) {
     if (h->K != K) return bfail(RN_ERR_STATE, "rn_batch_step: members have different precisions");
-    if (h->shape != b->tile) return bfail(RN_ERR_STATE, "rn_batch_step: a member's tile shape differs from the batch's");
+    if (h->shape != b->shape) return bfail(RN_ERR_STATE, "rn_batch_step: a member's tile shape differs from the batch's");
     if (!h->SA[0]) return bfail(RN_ERR_STATE, "rn_batch_step: a member has no buffers");
   }
   b->K = K;
@@ -585,8 +622,8 @@ int rn_batch_run(rn_batch b, const double* t_end, int chunk, long long max_steps
     for (size_t m = 0; m < nm; m++) {
       const rn_solver* h = b->members[m];
       if (b->runActive[m])
-        activeBlocks += ((h->Nx + TILE_TX[b->tile] - 1) / TILE_TX[b->tile]) *
-                        ((h->Nr + TILE_TY[b->tile] - 1) / TILE_TY[b->tile]);
+        activeBlocks += ((h->Nx + TILE_TX[b->shape] - 1) / TILE_TX[b->shape]) *
+                        ((h->Nr + TILE_TY[b->shape] - 1) / TILE_TY[b->shape]);
     }
     const int stoppedBlocks = tableBlocks - activeBlocks;
     if (stoppedBlocks >= b->numSMs && 8 * stoppedBlocks >= tableBlocks) {
@@ -730,10 +767,12 @@ int rn_batch_add(rn_batch b, rn_handle h, const rn_params* P, int* slot) {
     if (!(f == b->flags)) return bfail(RN_ERR_ARG, "rn_batch_add: physics flags (visc, chem, inj) differ from the batch's");
     if (h->K != b->members[0]->K) return bfail(RN_ERR_ARG, "rn_batch_add: precision differs from the batch's");
   }
-  if (h->tile != b->tile || h->shape != b->tile) {
-    int rc = rn_set_tile(h, b->tile);
+  {
+    const int rc = join_shape(b, h);
     if (rc != RN_OK) return rc;
   }
+  h->tile = b->tile;
+  h->autoShape = false;
   cudaEvent_t ev = nullptr;
   BCK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   if (b->members.empty()) b->flags = f;
@@ -782,27 +821,11 @@ int rn_batch_size(rn_batch b, int* members, long long* cells) {
 
 int rn_batch_set_tile(rn_batch b, int shape) {
   if (!b || shape < 0 || shape >= NTILES) return bfail(RN_ERR_ARG, "rn_batch_set_tile: bad argument");
-  if (shape == b->tile) return RN_OK;
-  BCK(cudaStreamSynchronize(b->stream));
-  const int old = b->tile;
-  for (size_t m = 0; m < b->members.size(); m++) {
-    rn_solver* h = b->members[m];
-    h->batch = nullptr;   // rn_set_tile refuses batch members
-    int rc = rn_set_tile(h, shape);
-    h->batch = b;
-    if (rc != RN_OK) {
-      std::string msg = rn_last_error();
-      for (size_t q = 0; q < m; q++) {
-        b->members[q]->batch = nullptr;
-        rn_set_tile(b->members[q], old);
-        b->members[q]->batch = b;
-      }
-      return bfail(rc, msg);
-    }
-  }
+  const int rc = use_shape(b, shape);
+  if (rc != RN_OK) return rc;
   b->tile = shape;
-  b->layout.clear();   // block table and descriptors are rebuilt by the next step
-  b->uploaded.clear();
+  b->autoShape = false;
+  for (rn_solver* h : b->members) h->tile = shape;
   return RN_OK;
 }
 
