@@ -268,12 +268,6 @@ RN_DEV Side side_of(float4 w, float4 b, float4 h, float4 g) {
 RN_DEV float4 half_slope4(float4 a, float4 b) {
   return cat4(half_slope2(lo2(a), lo2(b)), half_slope2(hi2(a), hi2(b)));
 }
-RN_DEV Side mirrored(float4 w, float4 b) {   // the cell's reflection in the face (normal velocity in .y)
-  Side o;
-  o.w = make_float4(w.x, -w.y, w.z, w.w);
-  o.s = b;
-  return o;
-}
 // |a - b| / min(a, b), a not NaN; 0 where b is NaN (a wall cell).
 RN_DEV float jump_ratio(float a, float b) {
   const float lo = fminf(a, b);
@@ -433,45 +427,59 @@ RN_DEV float hll_weight(float p1, float pa1, float pb1, float p2, float pa2, flo
 // Flux of the face between cells 1 and 2 of a line of four cells 0..3. DIR_R
 // selects the r-direction (normal velocity in .z): one instance of the code
 // serves both directions, since a second copy costs more in instruction-cache
-// misses than the selects cost in instructions. pa1, pb1, pa2, pb2: pressures
-// of the transverse neighbours of cells 1 and 2. A negative area makes the
-// face first order (next to a cut cell).
+// misses than the direction's selects cost in instructions. The reconstruction
+// works component by component, so only the two face states are turned into the
+// face-normal frame. pa1, pb1, pa2, pb2: pressures of the transverse
+// neighbours of cells 1 and 2. A negative area makes the face first order (next
+// to a cut cell). Walls and first-order faces are branches that most warps
+// skip, not selects that every face pays.
 RN_DEV Flux face_flux(bool DIR_R, float area, float4 w0, float4 b0, float4 w1, float4 b1, float4 w2, float4 b2,
                       float4 w3, float4 b3, float pa1, float pb1, float pa2, float pb2, const rn_params& P) {
-  const bool s0 = w0.x < 0.0f, s1 = w1.x < 0.0f, s2 = w2.x < 0.0f, s3 = w3.x < 0.0f;
-  if (s1 && s2) {
-    Flux out;
-    out.F = make_float4(0.f, 0.f, 0.f, 0.f);
-    out.Y = out.F;
-    out.O = 0.0f;
-    return out;
-  }
-  if (DIR_R) {   // face-normal frame: normal velocity in .y
-    float t;
-    t = w0.y; w0.y = w0.z; w0.z = t;
-    t = w1.y; w1.y = w1.z; w1.z = t;
-    t = w2.y; w2.y = w2.z; w2.z = t;
-    t = w3.y; w3.y = w3.z; w3.z = t;
-  }
+  const bool s1 = w1.x < 0.0f, s2 = w2.x < 0.0f;
   float hllw = 0.0f;
   Side L, R;
-  L.w = w1; L.s = b1; R.w = w2; R.s = b2;
-  if (s1 || s2) {
-    if (s1) L = mirrored(w2, b2);
-    else R = mirrored(w1, b1);
-  } else {
+  bool ok = false;
+  if (!(s1 || s2)) {
     hllw = hll_weight(w1.w, pa1, pb1, w2.w, pa2, pb2, P.hllBlend);
     if (P.order2 && area > 0.0f) {
       float4 d01 = diff4(w1, w0), d12 = diff4(w2, w1), d23 = diff4(w3, w2);
       float4 e01 = diff4(b1, b0), e12 = diff4(b2, b1), e23 = diff4(b3, b2);
-      // a wall neighbour is the cell's own reflection: the difference is twice
-      // the normal velocity, nothing else
-      if (s0) { d01 = make_float4(0.f, w1.y + w1.y, 0.f, 0.f); e01 = make_float4(0.f, 0.f, 0.f, 0.f); }
-      if (s3) { d23 = make_float4(0.f, -w2.y - w2.y, 0.f, 0.f); e23 = make_float4(0.f, 0.f, 0.f, 0.f); }
-      const Side tL = side_of<true>(w1, b1, half_slope4(d01, d12), half_slope4(e01, e12));
-      const Side tR = side_of<false>(w2, b2, half_slope4(d12, d23), half_slope4(e12, e23));
-      if (tL.w.x > 0.0f && tL.w.w > 0.0f && tR.w.x > 0.0f && tR.w.w > 0.0f) { L = tL; R = tR; }
+      const bool s0 = w0.x < 0.0f, s3 = w3.x < 0.0f;
+      if (__builtin_expect(s0 || s3, 0)) {
+        // a wall neighbour is the cell's own reflection: the difference is
+        // twice the normal velocity, nothing else
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s0) {
+          d01 = DIR_R ? make_float4(0.f, 0.f, w1.z + w1.z, 0.f) : make_float4(0.f, w1.y + w1.y, 0.f, 0.f);
+          e01 = z;
+        }
+        if (s3) {
+          d23 = DIR_R ? make_float4(0.f, 0.f, -w2.z - w2.z, 0.f) : make_float4(0.f, -w2.y - w2.y, 0.f, 0.f);
+          e23 = z;
+        }
+      }
+      L = side_of<true>(w1, b1, half_slope4(d01, d12), half_slope4(e01, e12));
+      R = side_of<false>(w2, b2, half_slope4(d12, d23), half_slope4(e12, e23));
+      ok = L.w.x > 0.0f && L.w.w > 0.0f && R.w.x > 0.0f && R.w.w > 0.0f;
     }
+  }
+  if (__builtin_expect(!ok, 0)) {                // first order, or a wall on one side
+    if (s1 && s2) {
+      Flux none;
+      none.F = make_float4(0.f, 0.f, 0.f, 0.f);
+      none.Y = none.F;
+      none.O = 0.0f;
+      return none;
+    }
+    L.w = s1 ? w2 : w1; L.s = s1 ? b2 : b1;
+    R.w = s2 ? w1 : w2; R.s = s2 ? b1 : b2;
+    if (s1) { if (DIR_R) L.w.z = -L.w.z; else L.w.y = -L.w.y; }
+    if (s2) { if (DIR_R) R.w.z = -R.w.z; else R.w.y = -R.w.y; }
+  }
+  if (DIR_R) {   // face-normal frame: normal velocity in .y
+    float t;
+    t = L.w.y; L.w.y = L.w.z; L.w.z = t;
+    t = R.w.y; R.w.y = R.w.z; R.w.z = t;
   }
   Flux out = hllc(L, R, hllw);
   if (DIR_R) { float t = out.F.y; out.F.y = out.F.z; out.F.z = t; }   // rotate momentum back to (x, r)

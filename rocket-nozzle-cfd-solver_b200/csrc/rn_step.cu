@@ -377,40 +377,81 @@ __device__ __forceinline__ void store_areas(const Grid& g, int x0, int y0, const
 }
 
 // FS_FLUX_X/R: every face of the tile (x-faces, then r-faces) and of its
-// listed members in one loop through one instance of the flux code. Face k's
-// 4 cells along the normal are primitive slots b, b + d, b + 2d, b + 3d and its
-// sensor cells (k1 +- t, ij +- t of makeFluxShader, solver.js:133-259)
-// b + d +- t and b + 2d +- t: tile faces have (d, t) = (1, PX) (x) or (PX, 1)
-// (r); a listed member's faces live in its 5x5 block, with 5 in place of PX.
-// One code path for every face also makes the fast precision's contracted
-// multiply-adds round alike in every tile shape.
+// listed members through one instance of the flux code. Face k's 4 cells along
+// the normal are primitive slots b, b + d, b + 2d, b + 3d and its sensor cells
+// (k1 +- t, ij +- t of makeFluxShader, solver.js:133-259) b + d +- t and
+// b + 2d +- t: tile faces have (d, t) = (1, PX) (x) or (PX, 1) (r); a listed
+// member's faces live in its 5x5 block, with 5 in place of PX. One code path
+// for every face also makes the fast precision's contracted multiply-adds
+// round alike in every tile shape.
 template <class T>
-__device__ __forceinline__ void inviscid_faces(const Grid& g, const rn_params& P, const int* xc, int xn,
-                                               const float4* sW, const float4* sWb, float4* sF, float4* sY,
-                                               float* sO, const float* sAr) {
+__device__ __forceinline__ void inviscid_face(int k, bool dirR, int b, int d, int t, const rn_params& P,
+                                              const float4* sW, const float4* sWb, float4* sF, float4* sY, float* sO,
+                                              const float* sAr) {
+  Flux f;
+  f.F = make_float4(0.f, 0.f, 0.f, 0.f); f.Y = f.F; f.O = 0.f;
+  const float area = sAr[k];   // the face's open area, 0 where it is not drawn
+  if (area != 0.0f)
+    f = face_flux(dirR, area, sW[b], sWb[b], sW[b + d], sWb[b + d], sW[b + 2 * d], sWb[b + 2 * d], sW[b + 3 * d],
+                  sWb[b + 3 * d], sW[b + d + t].w, sW[b + d - t].w, sW[b + 2 * d + t].w, sW[b + 2 * d - t].w, P);
+  sF[k] = f.F; sY[k] = f.Y; sO[k] = f.O;
+}
+// First slot of tile x-face k and r-face k - NXF.
+template <class T>
+__device__ __forceinline__ int xface_slot(int k) {
+  const int ly = k / (T::TX + 1), lx = k - ly * (T::TX + 1);
+  return (ly + 2) * T::PX + lx;
+}
+template <class T>
+__device__ __forceinline__ int rface_slot(int k) {
+  const int kk = k - T::NXF, ly = kk / T::TX, lx = kk - ly * T::TX;
+  return ly * T::PX + lx + 2;
+}
+// Face w of listed member e, q = 4e + w (W, E at mx + o; S, N at my + o).
+template <class T>
+__device__ __forceinline__ void member_face_slot(int q, bool& dirR, int& b, int& d, int& t) {
+  const int e = q >> 2, w = q & 3, o = w & 1;
+  dirR = w >= 2;
+  b = dirR ? ext_prim<T>(e, 0, o - 2) : ext_prim<T>(e, o - 2, 0);
+  d = dirR ? 5 : 1;
+  t = dirR ? 1 : 5;
+}
+template <class T>
+__device__ __forceinline__ void inviscid_faces(const rn_params& P, int xn, const float4* sW, const float4* sWb,
+                                               float4* sF, float4* sY, float* sO, const float* sAr) {
   constexpr int NXR = T::NXF + T::NRF;
-  for (int k = threadIdx.x; k < NXR + 4 * xn; k += T::NT) {
-    int b, d, t;
-    bool dirR;
-    if (k < T::NXF) {
-      const int ly = k / (T::TX + 1), lx = k - ly * (T::TX + 1);
-      b = (ly + 2) * T::PX + lx; d = 1; t = T::PX; dirR = false;
-    } else if (k < NXR) {
-      const int kk = k - T::NXF, ly = kk / T::TX, lx = kk - ly * T::TX;
-      b = ly * T::PX + lx + 2; d = T::PX; t = 1; dirR = true;
-    } else {                                     // member e's face w (W, E at mx + o; S, N at my + o)
-      const int q = k - NXR, e = q >> 2, w = q & 3, o = w & 1;
-      dirR = w >= 2;
-      b = dirR ? ext_prim<T>(e, 0, o - 2) : ext_prim<T>(e, o - 2, 0);
-      d = dirR ? 5 : 1; t = dirR ? 1 : 5;
+  if constexpr (T::WIDE || T::NXF > T::NT || T::NRF > T::NT) {
+    // one flat list
+    for (int k = threadIdx.x; k < NXR + 4 * xn; k += T::NT) {
+      int b, d, t;
+      bool dirR;
+      if (k < T::NXF) { b = xface_slot<T>(k); d = 1; t = T::PX; dirR = false; }
+      else if (k < NXR) { b = rface_slot<T>(k); d = T::PX; t = 1; dirR = true; }
+      else member_face_slot<T>(k - NXR, dirR, b, d, t);
+      inviscid_face<T>(k, dirR, b, d, t, P, sW, sWb, sF, sY, sO, sAr);
     }
-    Flux f;
-    f.F = make_float4(0.f, 0.f, 0.f, 0.f); f.Y = f.F; f.O = 0.f;
-    const float area = sAr[k];   // the face's open area, 0 where it is not drawn
-    if (area != 0.0f)
-      f = face_flux(dirR, area, sW[b], sWb[b], sW[b + d], sWb[b + d], sW[b + 2 * d], sWb[b + 2 * d], sW[b + 3 * d],
-                    sWb[b + 3 * d], sW[b + d + t].w, sW[b + d - t].w, sW[b + 2 * d + t].w, sW[b + 2 * d - t].w, P);
-    sF[k] = f.F; sY[k] = f.Y; sO[k] = f.O;
+  } else {
+    // a pass a direction and one for the members: the direction and the strides
+    // are the same across the block, which saves their selects (flat list ->
+    // passes, 16x15: viscous 2048x768 252 -> 248 us a step, plain 4096x1536
+    // 687 -> 680). Where a direction has more faces than the block threads
+    // (16x16) it would take more passes than the flat list, and the WIDE
+    // shapes' grids wait on a block's latency, which more passes lengthen
+    // (viscous 128x48 13.0 -> 14.3 us, 512x192 21.6 -> 23.1).
+#pragma unroll 1
+    for (int pass = 0; pass < (xn > 0 ? 3 : 2); pass++) {
+      const int k0 = pass == 0 ? 0 : pass == 1 ? T::NXF : NXR;
+      const int k1 = pass == 0 ? T::NXF : pass == 1 ? NXR : NXR + 4 * xn;
+#pragma unroll 1
+      for (int k = k0 + int(threadIdx.x); k < k1; k += T::NT) {
+        int b, d, t;
+        bool dirR;
+        if (pass == 0) { b = xface_slot<T>(k); d = 1; t = T::PX; dirR = false; }
+        else if (pass == 1) { b = rface_slot<T>(k); d = T::PX; t = 1; dirR = true; }
+        else member_face_slot<T>(k - NXR, dirR, b, d, t);
+        inviscid_face<T>(k, dirR, b, d, t, P, sW, sWb, sF, sY, sO, sAr);
+      }
+    }
   }
 }
 
@@ -590,7 +631,7 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
   load_prims<T>(g, a.A, a.B, t, P, x0, y0, xc, NP, RAW, sMask, sW, sWb);
   store_areas<T>(g, x0, y0, xc, xn, fa, sAr);
   __syncthreads();
-  inviscid_faces<T>(g, P, xc, xn, sW, sWb, sF, sY, sO, sAr);
+  inviscid_faces<T>(P, xn, sW, sWb, sF, sY, sO, sAr);
   __syncthreads();
 
   const int i = x0 + tid % TX, j = y0 + tid / TX;
@@ -878,7 +919,7 @@ __device__ __forceinline__ void stage2_physics_body(const StageArgs& a, const Ph
     float4* sF = R;
     float4* sY = sF + NF;
     float* sO = reinterpret_cast<float*>(sY + NF);
-    inviscid_faces<T>(g, P, xc, xn, sW, sWb, sF, sY, sO, sAr);
+    inviscid_faces<T>(P, xn, sW, sWb, sF, sY, sO, sAr);
     __syncthreads();
     // One flat list (T::WIDE): the stage-2 update of the tile's cells and of
     // its listed members, then FS_VCELL of the vcell slots. FS_VCELL reads only
