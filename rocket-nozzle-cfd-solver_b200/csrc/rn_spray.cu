@@ -121,26 +121,26 @@ __global__ void __launch_bounds__(256) k_parcels(SprayArgs a, rn_params P) {
         float dn = d, mn = m;
         if (w.x > 0.0f) {
           float rm = (1.0f - s.x) * P.gas[0] + s.y * P.Rs[0] + s.w * P.Rs[1] + fmaxf(s.x - s.y - s.w, 0.0f) * P.Rs[2];
-          float T = w.w / (w.x * rm) * P.gas[2];
+          float T = fdiv(w.w, w.x * rm) * P.gas[2];
           float rhoG = w.x * 1.225f, Urel = len2(w.y - vx, w.z - vy) * 287.6f + 1e-3f;
-          float mu = 1.458e-6f * T * sqrtf(T) / (T + 110.4f);
-          float Re = rhoG * Urel * d / mu;
-          float invTau = 18.0f * mu * (1.0f + 0.15f * powf(fminf(Re, 1000.0f), 0.687f)) / (pr[0] * d * d);
+          float mu = fdiv(1.458e-6f * T * sqrtf(T), T + 110.4f);
+          float Re = fdiv(rhoG * Urel * d, mu);
+          float invTau = fdiv(18.0f * mu * (1.0f + 0.15f * powf(fminf(Re, 1000.0f), 0.687f)), pr[0] * d * d);
           float e = expf(-dts * invTau);
           vx = w.y + (vx - w.y) * e;
           vy = w.z + (vy - w.z) * e;
           float cp = rm * 287.05f * (s.z + 1.0f);
-          float Bs = fmaxf(cp * (T - pr[1]), 0.0f) / pr[2];
-          float K = 8.0f * (mu / 0.7f) / pr[0] * logf(1.0f + Bs) * (1.0f + 0.27f * sqrtf(Re));
+          float Bs = fdiv(fmaxf(cp * (T - pr[1]), 0.0f), pr[2]);
+          float K = fdiv(8.0f * (mu / 0.7f), pr[0]) * logf(1.0f + Bs) * (1.0f + 0.27f * sqrtf(Re));
           float d2 = d * d - K * dts;
           dn = d2 > 1e-12f ? sqrtf(d2) : 0.0f;
-          float f = dn / d;
+          float f = fdiv(dn, d);
           mn = dn > 0.0f ? m * f * f * f : 0.0f;
-          float we = rhoG * Urel * Urel * dn / pr[3];
+          float we = fdiv(rhoG * Urel * Urel * dn, pr[3]);
           if (we > 12.0f && dn > 0.0f) {
-            float dst = 12.0f * pr[3] / (rhoG * Urel * Urel);
-            float tb = 3.0f * dn / Urel * sqrtf(pr[0] / rhoG);
-            dn = mixf(dn, fmaxf(dst, 2e-6f), 1.0f - expf(-dts / tb));
+            float dst = fdiv(12.0f * pr[3], rhoG * Urel * Urel);
+            float tb = fdiv(3.0f * dn, Urel) * sqrtf(fdiv(pr[0], rhoG));
+            dn = mixf(dn, fmaxf(dst, 2e-6f), 1.0f - expf(fdiv(-dts, tb)));
           }
         }
         float xi = pb.w;
@@ -301,9 +301,13 @@ __global__ void __launch_bounds__(256) k_apply(ApplyArgs a, rn_params P) {
 #ifdef RN_FAST
       const ulonglong2* c = reinterpret_cast<const ulonglong2*>(a.acc) + 2 * size_t(kh);
       const ulonglong2 c01 = c[0], c23 = c[1];
-      const float sm = dep_scale_mass(P, a.boundIn), sp = dep_scale_mom(P, a.boundIn);
-      float4 s = make_float4(from_fixed(c01.x, sm), from_fixed(c01.y, sm), from_fixed(c23.x, sp),
-                             from_fixed(c23.y, sp));
+      // most cells hold no deposits: the conversions (four FP64 quotients) and
+      // the scales are for those that do
+      float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+      if ((c01.x | c01.y | c23.x | c23.y) != 0ull) {
+        const float sm = dep_scale_mass(P, a.boundIn), sp = dep_scale_mom(P, a.boundIn);
+        s = make_float4(from_fixed(c01.x, sm), from_fixed(c01.y, sm), from_fixed(c23.x, sp), from_fixed(c23.y, sp));
+      }
 #else
       float4 s = a.src[kh];
 #endif
