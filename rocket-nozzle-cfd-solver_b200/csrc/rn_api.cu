@@ -254,9 +254,25 @@ int rn_build_tile_maps(rn_solver* h) {
   return RN_OK;
 }
 
-int rn_mask_refresh(rn_solver* h) {
-  CK(cudaMemcpy2DAsync(h->maskP, size_t(h->maskPitch), h->mask, size_t(h->Nx), size_t(h->Nx), size_t(h->Nr),
-                       cudaMemcpyDeviceToDevice, h->stream));
+__global__ void k_cell_classes(Grid g, uint8_t* __restrict__ out, int pitch) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+  if (i >= g.Nx) return;
+  const int k = j * g.Nx + i;
+  const float4 gm = g.geoM[k], gg = g.geoG[k], ga = g.geoA[j * (g.Nx + 1) + i];
+  const int z = __float2int_rn(gm.z);
+  const float row = float(j);
+  int c = g.mask[k] ? CELL_SOLID : 0;
+  if (!c && gm.x == 0.0f && gm.y == 0.0f && (z & 15) == 0 && gg.x == row + 0.5f && gg.y == 1.0f && gg.z == 0.0f &&
+      gg.w == 0.0f)
+    c |= CELL_PLAIN;
+  if (!(z & 16)) c |= CELL_NO_BAND;
+  if (gm.w == TURB_L0) c |= CELL_L0;
+  if (ga.z == row + 0.5f && ga.w == row) c |= CELL_FACES;
+  out[size_t(j) * pitch + i] = uint8_t(c);
+}
+int rn_classes_refresh(rn_solver* h) {
+  k_cell_classes<<<dim3((h->Nx + 127) / 128, h->Nr), 128, 0, h->stream>>>(h->grid(), h->maskP, h->maskPitch);
+  CK(cudaGetLastError());
   return RN_OK;
 }
 
@@ -510,7 +526,7 @@ int rn_set_mask(rn_handle h, const uint8_t* mask) {
   for (size_t k = 0; k < N; k++) m[k] = mask[k] ? 1 : 0;
   CK(cudaMemcpyAsync(h->mask, m.data(), N, cudaMemcpyHostToDevice, h->stream));
   {
-    const int rc = rn_mask_refresh(h);
+    const int rc = rn_classes_refresh(h);
     if (rc != RN_OK) return rc;
   }
   CK(cudaStreamSynchronize(h->stream));
@@ -563,6 +579,8 @@ int rn_set_geometry(rn_handle h, const uint8_t* mask, const float* geoA, const f
   CK(cudaMemcpyAsync(h->geoG, geoG, sizeof(float4) * N, cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->geoM, geoM, sizeof(float4) * N, cudaMemcpyHostToDevice, h->stream));
   if (jWall) CK(cudaMemcpyAsync(h->jw, jWall, sizeof(float4) * Nx, cudaMemcpyHostToDevice, h->stream));
+  rc = rn_classes_refresh(h);
+  if (rc != RN_OK) return rc;
   CK(cudaStreamSynchronize(h->stream));
   return RN_OK;
 }

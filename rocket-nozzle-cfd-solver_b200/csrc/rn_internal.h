@@ -41,8 +41,9 @@ struct rn_solver {
   int cur = 0;
   float4 *geoA = nullptr, *geoG = nullptr, *geoM = nullptr, *jw = nullptr, *wallRow = nullptr;
   uint8_t* mask = nullptr;
-  // the mask again with rows padded to 16 bytes (a tensor map's row stride
-  // must be a multiple of 16 bytes), refreshed whenever the mask changes
+  // the cells' classes (CellClass), rows padded to 16 bytes (a tensor map's row
+  // stride must be a multiple of 16 bytes), rebuilt whenever the mask or the
+  // geometry changes
   uint8_t* maskP = nullptr;
   int maskPitch = 0;
   // tensor maps of the stage kernels' halo copies, one TileMaps per tile shape
@@ -135,8 +136,8 @@ struct rn_solver {
 int rn_build_tile_maps(rn_solver* h);
 // Destroy h's step graphs (their launches name its buffers and lists).
 void rn_drop_step_graphs(rn_solver* h);
-// Copy h->mask into its row-pitched copy (queued on h->stream).
-int rn_mask_refresh(rn_solver* h);
+// Rebuild h's cell classes from its mask and geometry (queued on h->stream).
+int rn_classes_refresh(rn_solver* h);
 // Record an error for rn_last_error() and return `code`.
 int rn_record_error(int code, const std::string& msg);
 int rn_record_cuda(cudaError_t e, const char* what);

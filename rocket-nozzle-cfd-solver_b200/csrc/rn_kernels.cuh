@@ -41,6 +41,19 @@ inline int tile_count(int shape, int Nx, int Nr) {
 // batched 128x48 (2048 / 1536) 108 / 97; 1024x384 (1664 / 1536) 67.8 / 72.3, 24
 // batched mixed grids (2224 / 2040 a set of four) 622 / 694.
 inline bool prefer_16x16(long long tiles16x16, long long tiles16x15) { return 11 * tiles16x16 <= 10 * tiles16x15; }
+// A cell's class byte, in the row-pitched plane that the step kernels copy with
+// the halo (0 outside the grid). Almost all cells are uncut (99 % of the plume
+// and engine grids): their geometry is that of the grid, so the kernels form it
+// from the row instead of reading geoA, geoG and geoM (49 of the 113 bytes a
+// cell that stage 1 needs otherwise).
+enum CellClass : unsigned char {
+  CELL_SOLID = 1,
+  CELL_PLAIN = 2,     // fluid, its own group alone, geoG = (j + 1/2, 1, 0, 0): no wall, whole cell
+  CELL_NO_BAND = 4,   // not in the boundary-layer band (geoM.z bit 16)
+  CELL_L0 = 8,        // turbulence length TURB_L0
+  CELL_FACES = 16     // west and south face fully open: areas j + 1/2 and j, second order
+};
+constexpr float TURB_L0 = 0.17f;
 // Most out-of-tile group members one tile may list (set_geometry rejects more).
 constexpr int MAXX = 64;
 // Tiles listing more out-of-tile members than this run the fused stage-2 +

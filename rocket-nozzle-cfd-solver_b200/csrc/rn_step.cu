@@ -260,8 +260,15 @@ struct CellSrc {
     return T::WIDE && unsigned(i - x0) < unsigned(T::TX) && unsigned(j - y0) < unsigned(T::TY);
   }
   __device__ __forceinline__ int hslot(int i, int j) const { return (j - y0 + 2) * T::PX + (i - x0 + 2); }
-  __device__ __forceinline__ bool solid(int i, int j) const {
-    return in_halo(i, j) ? m[(j - y0 + 2) * T::MW + mo + (i - x0 + 2)] != 0 : g.mask[j * g.Nx + i] != 0;
+  // the cell's class; of a cell outside the staged block only whether it is
+  // solid, and so for WIDE shapes, which have the geometry staged (the classes
+  // cost viscous 128x48 2 %, 512x192 1 %)
+  __device__ __forceinline__ int cls(int i, int j) const {
+    if (unsigned(i - x0 + 2) < unsigned(T::PX) && unsigned(j - y0 + 2) < unsigned(T::PY)) {
+      const int c = m[(j - y0 + 2) * T::MW + mo + (i - x0 + 2)];
+      return T::WIDE ? c & CELL_SOLID : c;
+    }
+    return g.mask[j * g.Nx + i] != 0 ? CELL_SOLID : 0;
   }
   __device__ __forceinline__ float4 a(int i, int j) const { return in_halo(i, j) ? raw[hslot(i, j)] : A[j * g.Nx + i]; }
   __device__ __forceinline__ float4 b(int i, int j) const {
@@ -301,7 +308,7 @@ struct HaloCells {
   }
   __device__ __forceinline__ int slot(int i, int j) const { return (j - y0 + 2) * T::PX + (i - x0 + 2); }
   __device__ __forceinline__ bool solid(int i, int j) const {
-    return staged(i, j) ? m[(j - y0 + 2) * T::MW + mo + (i - x0 + 2)] != 0 : g.mask[j * g.Nx + i] != 0;
+    return staged(i, j) ? (m[(j - y0 + 2) * T::MW + mo + (i - x0 + 2)] & CELL_SOLID) != 0 : g.mask[j * g.Nx + i] != 0;
   }
   __device__ __forceinline__ float4 a(int i, int j) const { return staged(i, j) ? rA[slot(i, j)] : A[j * g.Nx + i]; }
   __device__ __forceinline__ float4 b(int i, int j) const { return staged(i, j) ? rB[slot(i, j)] : B[j * g.Nx + i]; }
@@ -330,7 +337,7 @@ __device__ __forceinline__ void load_prims(const Grid& g, const float4* __restri
       // a slot of the staged block is its own cell k of it (no lookup)
       const bool own = k < T::NPT;
       const float4 a = own ? R[k] : cells.a(i, j), b = own ? R[T::NPT8 + k] : cells.b(i, j);
-      const bool solid = own ? sMask[ly * T::MW + mo + lx] != 0 : cells.solid(i, j);
+      const bool solid = own ? (sMask[ly * T::MW + mo + lx] & CELL_SOLID) != 0 : cells.solid(i, j);
       if (solid) {
         W = wall_prim();
         Wb = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -349,30 +356,42 @@ __device__ __forceinline__ void load_prims(const Grid& g, const float4* __restri
   }
 }
 
-// Face areas into sAr: a thread's first x- and r-face (loaded at block start,
-// their latency hidden behind the halo copy), the rest of the tile's faces
-// (shapes with more faces than threads), then the listed members' faces.
+// Face areas into sAr, the tile's then the listed members'. WIDE shapes, whose
+// blocks' latency counts, load a thread's first x- and r-face at block start,
+// behind the halo copy. The others take the areas of fully open faces from the
+// staged classes and load only the rest (cut cells, the grid's far edges).
 struct FirstAreas {
   float x, r;
 };
 template <class T>
 __device__ __forceinline__ FirstAreas first_areas(const Grid& g, int x0, int y0) {
-  FirstAreas f;
-  const int tid = threadIdx.x;
-  f.x = tid < T::NXF ? xface_area<T>(g, tid, x0, y0) : 0.0f;
-  f.r = tid < T::NRF ? rface_area<T>(g, tid, x0, y0) : 0.0f;
+  FirstAreas f = {0.0f, 0.0f};
+  if constexpr (T::WIDE) {
+    const int tid = threadIdx.x;
+    if (tid < T::NXF) f.x = xface_area<T>(g, tid, x0, y0);
+    if (tid < T::NRF) f.r = rface_area<T>(g, tid, x0, y0);
+  }
   return f;
 }
 template <class T>
 __device__ __forceinline__ void store_areas(const Grid& g, int x0, int y0, const int* xc, int xn, FirstAreas f,
-                                            float* sAr) {
+                                            const uint8_t* sMask, float* sAr) {
   const int tid = threadIdx.x;
-  if (tid < T::NXF) sAr[tid] = f.x;
-  if (tid < T::NRF) sAr[T::NXF + tid] = f.r;
-  if constexpr (T::NXF > T::NT)
-    for (int k = tid + T::NT; k < T::NXF; k += T::NT) sAr[k] = xface_area<T>(g, k, x0, y0);
-  if constexpr (T::NRF > T::NT)
-    for (int k = tid + T::NT; k < T::NRF; k += T::NT) sAr[T::NXF + k] = rface_area<T>(g, k, x0, y0);
+  if constexpr (T::WIDE) {
+    if (tid < T::NXF) sAr[tid] = f.x;
+    if (tid < T::NRF) sAr[T::NXF + tid] = f.r;
+    static_assert(T::NXF <= T::NT && T::NRF <= T::NT, "a face of each direction a thread");
+  } else {
+    const uint8_t* m = sMask + 2 * T::MW + ((x0 - 2) - ((x0 - 2) & ~15)) + 2;   // class of the tile's first cell
+    for (int k = tid; k < T::NXF; k += T::NT) {
+      const int ly = k / (T::TX + 1), lx = k - ly * (T::TX + 1);
+      sAr[k] = (m[ly * T::MW + lx] & CELL_FACES) ? float(y0 + ly) + 0.5f : xface_area<T>(g, k, x0, y0);
+    }
+    for (int k = tid; k < T::NRF; k += T::NT) {
+      const int ly = k / T::TX, lx = k - ly * T::TX;
+      sAr[T::NXF + k] = (m[ly * T::MW + lx] & CELL_FACES) ? float(y0 + ly) : rface_area<T>(g, k, x0, y0);
+    }
+  }
   for (int q = tid; q < 4 * xn; q += T::NT) sAr[T::NXF + T::NRF + q] = member_face_area(g, q, xc);
 }
 
@@ -497,22 +516,30 @@ __device__ __forceinline__ bool update_cell(const StageArgs& a, const CellSrc<T>
   const Grid& g = a.g;
   const int Nx = g.Nx;
   const int k = j * Nx + i;
-  // the cell's own operands in one round of loads; a slave cell (host kh != k)
-  // then loads its host's
-  const bool solid = cs.solid(i, j);
-  const float4 gm = cs.gm(i, j), gg = cs.gg(i, j);
   float4 A = cs.a(i, j), B = cs.b(i, j), A0 = STAGE == 2 ? a.A0[k] : A, B0 = STAGE == 2 ? a.B0[k] : B;
-  if (solid) {
+  const int cl = cs.cls(i, j);
+  if (cl & CELL_SOLID) {
     oA = make_float4(P.ambCons[0], P.ambCons[1], P.ambCons[2], P.ambCons[3]);
     oB = make_float4(P.ambB[0], P.ambB[1], P.ambB[2], P.ambB[3]);
     return false;
   }
-  const int Hx = i + iround(gm.x), Hy = j + iround(gm.y), kh = Hy * Nx + Hx;
-  float ghz = gm.z;
-  if (kh != k) {
-    A = cs.a(Hx, Hy); B = cs.b(Hx, Hy);
-    if (STAGE == 2) { A0 = a.A0[kh]; B0 = a.B0[kh]; }
-    ghz = cs.gm(Hx, Hy).z;
+  // an uncut cell's geometry is the grid's; a slave cell (host kh != k) loads
+  // its host's operands
+  float4 gg = make_float4(float(j) + 0.5f, 1.0f, 0.0f, 0.0f);
+  float ghz = 0.0f;
+  int Hx = i, Hy = j;
+  if (!(cl & CELL_PLAIN)) {
+    const float4 gm = cs.gm(i, j);
+    gg = cs.gg(i, j);
+    Hx = i + iround(gm.x);
+    Hy = j + iround(gm.y);
+    ghz = gm.z;
+    const int kh = Hy * Nx + Hx;
+    if (kh != k) {
+      A = cs.a(Hx, Hy); B = cs.b(Hx, Hy);
+      if (STAGE == 2) { A0 = a.A0[kh]; B0 = a.B0[kh]; }
+      ghz = cs.gm(Hx, Hy).z;
+    }
   }
   // the host's primitives: it lies within a cell of the tile, so the primitive
   // phase left them in its halo slot (the same floats as to_prim's)
@@ -527,7 +554,7 @@ __device__ __forceinline__ bool update_cell(const StageArgs& a, const CellSrc<T>
   if (P.inj) group_flux<T, true>(Hx, Hy, sm_, x0, y0, xc, xn, Nx, sF, sY, sO, sAr, L, LY, LO);
   else group_flux<T, false>(Hx, Hy, sm_, x0, y0, xc, xn, Nx, sF, sY, sO, sAr, L, LY, LO);
   // embedded wall: pressure force along the r-weighted wall vector
-  float wl = len2(gg.z, gg.w);
+  const float wl = (cl & CELL_PLAIN) ? 0.0f : len2(gg.z, gg.w);
   if (wl > 1e-6f) {
     const Over per_wl = over(wl);
     float nx = per_wl(gg.z), nr = per_wl(gg.w);
@@ -629,7 +656,7 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
   __syncthreads();
   if (!halo_wait(bar, a.err)) return;
   load_prims<T>(g, a.A, a.B, t, P, x0, y0, xc, NP, RAW, sMask, sW, sWb);
-  store_areas<T>(g, x0, y0, xc, xn, fa, sAr);
+  store_areas<T>(g, x0, y0, xc, xn, fa, sMask, sAr);
   __syncthreads();
   inviscid_faces<T>(P, xn, sW, sWb, sF, sY, sO, sAr);
   __syncthreads();
@@ -670,7 +697,8 @@ __device__ __forceinline__ void vcell_at(const Grid& g, const CellSrc<T>& cs, co
   }
   float4 T1 = make_float4(0.f, 0.f, 0.f, 0.f), T2 = T1;
   if (i >= 0 && i < Nx && j >= 0 && j < Nr)
-    vcell(sW[c], sWb[c], sW[c + 1], sW[c - 1], sW[c + rs], sW[c - rs], i, j, cs.gm(i, j).w, dt, P, T1, T2);
+    vcell(sW[c], sWb[c], sW[c + 1], sW[c - 1], sW[c + rs], sW[c - rs], i, j,
+          (cs.cls(i, j) & CELL_L0) ? TURB_L0 : cs.gm(i, j).w, dt, P, T1, T2);
   sT1[k] = T1;
   sT2[k] = T2;
 }
@@ -734,14 +762,21 @@ __device__ __forceinline__ bool source_cell(const Grid& g, const CellSrc<T>& cs,
   constexpr int TW = T::TW;
   const int Nx = g.Nx, Nr = g.Nr;
   const int k = j * Nx + i;
-  const bool solid = cs.solid(i, j);
-  const float4 gmij = cs.gm(i, j), gg = cs.gg(i, j);
-  if (solid) {
+  const int cl = cs.cls(i, j);
+  if (cl & CELL_SOLID) {
     oA = make_float4(P.ambCons[0], P.ambCons[1], P.ambCons[2], P.ambCons[3]);
     oB = make_float4(P.ambB[0], P.ambB[1], P.ambB[2], P.ambB[3]);
     return false;
   }
-  const int Hx = i + iround(gmij.x), Hy = j + iround(gmij.y), kh = Hy * Nx + Hx;
+  float4 gg = make_float4(float(j) + 0.5f, 1.0f, 0.0f, 0.0f);
+  int Hx = i, Hy = j, sm_ = (cl & CELL_NO_BAND) ? 0 : 16;   // slave and band bits of an uncut cell
+  if (!(cl & CELL_PLAIN)) {
+    const float4 gmij = cs.gm(i, j);
+    gg = cs.gg(i, j);
+    Hx = i + iround(gmij.x);
+    Hy = j + iround(gmij.y);
+    sm_ = iround(Hy * Nx + Hx == k ? gmij.z : cs.gm(Hx, Hy).z);
+  }
   Prim q = to_prim(A, B);
   float rho = q.w.x, p = q.w.w, G = q.s.z;
   float velx = q.w.y, vely = q.w.z;
@@ -751,14 +786,13 @@ __device__ __forceinline__ bool source_cell(const Grid& g, const CellSrc<T>& cs,
   const int vh = (Hy - y0 + 1) * TW + (Hx - x0 + 1);
   float4 T1h = sT1[vh], T2h = sT2[vh];
   if (P.visc) {
-    const int sm_ = iround(kh == k ? gmij.z : cs.gm(Hx, Hy).z);
     float LO = 0.0f;
     group_flux<T, false>(Hx, Hy, sm_, x0, y0, xc, xn, Nx, sF, sY, nullptr, sAr, L, LY, LO);
     // axisymmetric hoop stress
     float r = fdiv(V, fmaxf(gg.y, 1e-6f)), vor = fdiv(vely, r);
     L.z -= T2h.x * (2.0f * vor - 0.6666667f * (T1h.x + T1h.w + vor)) * gg.y;
     // Werner-Wengle wall shear and Reynolds-analogy heat flux
-    float wl = len2(gg.z, gg.w);
+    const float wl = (cl & CELL_PLAIN) ? 0.0f : len2(gg.z, gg.w);
     if (wl > 1e-6f) {
       const Over per_wl = over(wl);
       float nx = per_wl(gg.z), nr = per_wl(gg.w);
@@ -913,7 +947,7 @@ __device__ __forceinline__ void stage2_physics_body(const StageArgs& a, const Ph
   __syncthreads();
   if (!halo_wait(bar, a.err)) return;
   load_prims<T>(g, a.A, a.B, t, P, x0, y0, xc, NP, RAW, sMask, sW, sWb);
-  store_areas<T>(g, x0, y0, xc, xn, fa, sAr);
+  store_areas<T>(g, x0, y0, xc, xn, fa, sMask, sAr);
   __syncthreads();
   {
     float4* sF = R;
@@ -960,9 +994,14 @@ __device__ __forceinline__ void stage2_physics_body(const StageArgs& a, const Ph
     const int k = j * Nx + i;
     float4 oA, oB, A = make_float4(0.f, 0.f, 0.f, 0.f), B = A;
     float Bw = 0.0f;
-    if (!cs.solid(i, j)) {
-      float4 gm = cs.gm(i, j);
-      const int Hx = i + iround(gm.x), Hy = j + iround(gm.y);
+    const int cl = cs.cls(i, j);
+    if (!(cl & CELL_SOLID)) {
+      int Hx = i, Hy = j;
+      if (!(cl & CELL_PLAIN)) {
+        const float4 gm = cs.gm(i, j);
+        Hx = i + iround(gm.x);
+        Hy = j + iround(gm.y);
+      }
       const int hx = Hx - x0, hy = Hy - y0;
       int s;
       if (unsigned(hx) < unsigned(TX) && unsigned(hy) < unsigned(T::TY)) {

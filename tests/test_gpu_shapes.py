@@ -52,3 +52,54 @@ def test_resize_follows_the_default_shape(rn):
     out = g.readAll()
     assert np.array_equal(out["A"], ref[0]["A"]) and np.array_equal(out["B"], ref[0]["B"])
     g.close()
+
+
+@pytest.mark.parametrize("kind", ["viscous_plume", "plain_small"])
+@pytest.mark.parametrize("tile", ["16x15", "16x16", "16x8", "32x15", None])
+def test_cell_classes_follow_the_geometry(rn, oracle, kind, tile):
+    """The step kernels take uncut cells' volumes, areas and turbulence lengths
+    from the cell classes instead of the geometry planes. A geometry with
+    values off the grid's own in single cells and faces (each class bit on and
+    off, alone and together, at tile and grid edges, zeros of either sign) steps
+    bit for bit as the 14x16 shape steps it in exact precision, which reads the
+    planes, and as the oracle but for the wall functions' pow (last bits, 6e-8
+    of a wall cell's terms in each of 9 steps: 1e-6); so does the grid's own
+    geometry set after it."""
+    from helpers import state_rel_l2
+    from rocket_nozzle_cfd_solver_b200 import configs
+    s = rn.build_sim_setup(getattr(configs, kind)(77, 33)[0])
+    Nx, Nr = s.Nx, s.Nr
+    rng = np.random.default_rng(11)
+    geo = dict(s.geo)
+    gA, gG, gM = (np.array(geo[k], np.float32) for k in ("geoA", "geoG", "geoM"))
+    gA, gG, gM = gA.reshape(Nr + 1, Nx + 1, 4), gG.reshape(Nr, Nx, 4), gM.reshape(Nr, Nx, 4)
+    pick = lambda p, sh: rng.uniform(size=sh) < p  # noqa: E731
+    for k in (2, 3):
+        gA[..., k] = np.where(pick(0.05, gA.shape[:2]), gA[..., k] * np.float32(0.9), gA[..., k])
+        gA[..., k] = np.where(pick(0.05, gA.shape[:2]), -gA[..., k], gA[..., k])
+    for k in (0, 1):
+        gG[..., k] = np.where(pick(0.05, (Nr, Nx)), gG[..., k] * np.float32(1.1), gG[..., k])
+    for k in (2, 3):
+        gG[..., k] = np.where(pick(0.02, (Nr, Nx)), np.float32(0.2), gG[..., k])
+        gG[..., k] = np.where(pick(0.05, (Nr, Nx)) & (gG[..., k] == 0), np.float32(-0.0), gG[..., k])
+    gM[..., 3] = np.where(pick(0.1, (Nr, Nx)), np.float32(0.25), gM[..., 3])
+    gM[..., 2] = np.where(pick(0.05, (Nr, Nx)) & (gM[..., 2] == 0), np.float32(16.0), gM[..., 2])
+    geo.update(geoA=gA.reshape(-1), geoG=gG.reshape(-1), geoM=gM.reshape(-1))
+    init = s.initialState()
+    g, ref = rn.GPUSolver(Nx, Nr), rn.GPUSolver(Nx, Nr)
+    for h in (g, ref):
+        h.setPrecision("exact")
+    if tile:
+        g.setTile(tile)
+    ref.setTile("14x16")
+    for planes in (geo, s.geo):
+        o = oracle.OracleSolver(Nx, Nr)
+        for h in (g, ref, o):
+            h.setGeometry(planes)
+            h.setState(init["A"], init["B"])
+            h.step(9, s.P)
+        a, b = g.readAll(), ref.readAll()
+        assert np.array_equal(a["A"], b["A"]) and np.array_equal(a["B"], b["B"])
+        assert max(state_rel_l2(a, o.readAll()).values()) <= 1e-6
+    g.close()
+    ref.close()
