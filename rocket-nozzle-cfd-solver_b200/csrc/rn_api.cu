@@ -268,6 +268,9 @@ __global__ void k_cell_classes(Grid g, uint8_t* __restrict__ out, int pitch) {
   if (!(z & 16)) c |= CELL_NO_BAND;
   if (gm.w == TURB_L0) c |= CELL_L0;
   if (ga.z == row + 0.5f && ga.w == row) c |= CELL_FACES;
+  const float east = g.geoA[j * (g.Nx + 1) + i + 1].z, north = g.geoA[(j + 1) * (g.Nx + 1) + i].w;
+  if (fabsf(ga.z) == row + 0.5f && fabsf(ga.w) == row && fabsf(east) == row + 0.5f && fabsf(north) == row + 1.0f)
+    c |= CELL_BOX;
   out[size_t(j) * pitch + i] = uint8_t(c);
 }
 int rn_classes_refresh(rn_solver* h) {

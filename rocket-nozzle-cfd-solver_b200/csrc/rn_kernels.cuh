@@ -51,7 +51,8 @@ enum CellClass : unsigned char {
   CELL_PLAIN = 2,     // fluid, its own group alone, geoG = (j + 1/2, 1, 0, 0): no wall, whole cell
   CELL_NO_BAND = 4,   // not in the boundary-layer band (geoM.z bit 16)
   CELL_L0 = 8,        // turbulence length TURB_L0
-  CELL_FACES = 16     // west and south face fully open: areas j + 1/2 and j, second order
+  CELL_FACES = 16,    // west and south face fully open: areas j + 1/2 and j, second order
+  CELL_BOX = 32       // all four faces of the size of the grid's, whatever their sign
 };
 constexpr float TURB_L0 = 0.17f;
 // Most out-of-tile group members one tile may list (set_geometry rejects more).

@@ -505,6 +505,24 @@ RN_DEV void sub4(float4& L, float ae, float4 fe, float aw, float4 fw) {
   L.w -= ae * fe.w - aw * fw.w;
 }
 
+// L of a cell whose x-faces have area ax and whose south and north faces have
+// areas as_ and as_ + 1 (an uncut cell), after sub4's of both directions from
+// L = 0. The fast variant forms the differences first: two packed operations a
+// pair for x, three for r, where sub4 takes twelve scalar ones.
+RN_DEV float4 box4(float ax, float as_, float4 fw, float4 fe, float4 fs, float4 fn) {
+#ifdef RN_FAST
+  const float2 x = make_float2(-ax, -ax), r = make_float2(as_, as_);
+  const float2 xl = mul2(x, sub2(lo2(fe), lo2(fw))), xh = mul2(x, sub2(hi2(fe), hi2(fw)));
+  const float2 rl = madd2(r, sub2(lo2(fn), lo2(fs)), lo2(fn)), rh = madd2(r, sub2(hi2(fn), hi2(fs)), hi2(fn));
+  return cat4(sub2(xl, rl), sub2(xh, rh));
+#else
+  float4 L = make_float4(0.f, 0.f, 0.f, 0.f);
+  sub4(L, ax, fe, ax, fw);
+  sub4(L, as_ + 1.0f, fn, as_, fs);
+  return L;
+#endif
+}
+
 // GLSL_GAS (solver.js:445-450)
 RN_DEV float sutherland(float TK, const rn_params& P) { return fdiv(P.gas[3] * 1.458e-6f * TK * sqrtf(TK), TK + 110.4f); }
 RN_DEV float rmix(float4 s, const rn_params& P) {

@@ -506,6 +506,45 @@ __device__ __forceinline__ void group_flux(int Hx, int Hy, int sm_, int x0, int 
   }
 }
 
+// group_flux of a tile cell that is its own group and has the grid's own face
+// sizes (CELL_PLAIN and CELL_BOX): its four faces directly.
+template <class T, bool WITH_O>
+__device__ __forceinline__ void box_flux(int i, int j, int x0, int y0, const float4* sF, const float4* sY,
+                                         const float* sO, float4& L, float4& LY, float& LO) {
+  const int mx = i - x0, my = j - y0, fw = my * (T::TX + 1) + mx, fs = T::NXF + my * T::TX + mx;
+  const float as_ = float(j), ax = as_ + 0.5f;
+  L = box4(ax, as_, sF[fw], sF[fw + 1], sF[fs], sF[fs + T::TX]);
+  LY = box4(ax, as_, sY[fw], sY[fw + 1], sY[fs], sY[fs + T::TX]);
+  if constexpr (WITH_O) {
+    LO -= ax * sO[fw + 1] - ax * sO[fw];
+    LO -= (as_ + 1.0f) * sO[fs + T::TX] - as_ * sO[fs];
+  }
+}
+// whether a cell of class cl, in the tile, takes box_flux
+template <class T>
+__device__ __forceinline__ bool box_cell(int cl, int i, int j, int x0, int y0) {
+  return !T::WIDE && (cl & (CELL_PLAIN | CELL_BOX)) == (CELL_PLAIN | CELL_BOX) && unsigned(i - x0) < unsigned(T::TX) &&
+         unsigned(j - y0) < unsigned(T::TY);
+}
+
+// The RK combination: U + f L in stage 1, 0.5 (U0 + U + f L) in stage 2.
+// PACKED (fast variant): in lane pairs, half the instructions; the WIDE shapes
+// keep the scalar form, whose chains are shorter (viscous 512x192 21.6 against
+// 22.0 us).
+template <int STAGE, bool PACKED>
+__device__ __forceinline__ float4 rk_combine(float f, float4 L, float4 U, float4 U0) {
+#ifdef RN_FAST
+  if constexpr (PACKED) {
+    const float2 ff = make_float2(f, f), h = make_float2(0.5f, 0.5f);
+    if (STAGE == 1) return cat4(madd2(ff, lo2(L), lo2(U)), madd2(ff, hi2(L), hi2(U)));
+    return cat4(mul2(h, madd2(ff, lo2(L), add2(lo2(U0), lo2(U)))), mul2(h, madd2(ff, hi2(L), add2(hi2(U0), hi2(U)))));
+  }
+#endif
+  if (STAGE == 1) return make_float4(U.x + f * L.x, U.y + f * L.y, U.z + f * L.z, U.w + f * L.w);
+  return make_float4(0.5f * (U0.x + U.x + f * L.x), 0.5f * (U0.y + U.y + f * L.y), 0.5f * (U0.z + U.z + f * L.z),
+                     0.5f * (U0.w + U.w + f * L.w));
+}
+
 // FS_UPDATE of cell (i, j) inside the grid: the RK update of its host's
 // cut-cell group. Returns whether the cell is fluid.
 template <class T, int STAGE>
@@ -551,7 +590,10 @@ __device__ __forceinline__ bool update_cell(const StageArgs& a, const CellSrc<T>
   float4 L = make_float4(0.f, 0.f, 0.f, 0.f), LY = L;
   float LO = 0.0f;
   const int sm_ = iround(ghz);
-  if (P.inj) group_flux<T, true>(Hx, Hy, sm_, x0, y0, xc, xn, Nx, sF, sY, sO, sAr, L, LY, LO);
+  if (box_cell<T>(cl, i, j, x0, y0)) {
+    if (P.inj) box_flux<T, true>(i, j, x0, y0, sF, sY, sO, L, LY, LO);
+    else box_flux<T, false>(i, j, x0, y0, sF, sY, sO, L, LY, LO);
+  } else if (P.inj) group_flux<T, true>(Hx, Hy, sm_, x0, y0, xc, xn, Nx, sF, sY, sO, sAr, L, LY, LO);
   else group_flux<T, false>(Hx, Hy, sm_, x0, y0, xc, xn, Nx, sF, sY, sO, sAr, L, LY, LO);
   // embedded wall: pressure force along the r-weighted wall vector
   const float wl = (cl & CELL_PLAIN) ? 0.0f : len2(gg.z, gg.w);
@@ -566,16 +608,7 @@ __device__ __forceinline__ bool update_cell(const StageArgs& a, const CellSrc<T>
   float invV = fdiv(1.0f, fmaxf(gg.x, 1e-6f));
   float4 LB = make_float4(LY.x, LY.y, LY.z - q.s.z * LY.w, LO);
   float f = dt * invV;
-  float4 U, UY;
-  if (STAGE == 1) {
-    U = make_float4(A.x + f * L.x, A.y + f * L.y, A.z + f * L.z, A.w + f * L.w);
-    UY = make_float4(B.x + f * LB.x, B.y + f * LB.y, B.z + f * LB.z, B.w + f * LB.w);
-  } else {
-    U = make_float4(0.5f * (A0.x + A.x + f * L.x), 0.5f * (A0.y + A.y + f * L.y), 0.5f * (A0.z + A.z + f * L.z),
-                    0.5f * (A0.w + A.w + f * L.w));
-    UY = make_float4(0.5f * (B0.x + B.x + f * LB.x), 0.5f * (B0.y + B.y + f * LB.y),
-                     0.5f * (B0.z + B.z + f * LB.z), 0.5f * (B0.w + B.w + f * LB.w));
-  }
+  const float4 U = rk_combine<STAGE, !T::WIDE>(f, L, A, A0), UY = rk_combine<STAGE, !T::WIDE>(f, LB, B, B0);
   float rho = fmaxf(U.x, RHO_MIN);
   const Over per_den = over(fmaxf(U.x, RHO_MIN));
   float vx = per_den(U.y), vy = per_den(U.z);
@@ -787,7 +820,8 @@ __device__ __forceinline__ bool source_cell(const Grid& g, const CellSrc<T>& cs,
   float4 T1h = sT1[vh], T2h = sT2[vh];
   if (P.visc) {
     float LO = 0.0f;
-    group_flux<T, false>(Hx, Hy, sm_, x0, y0, xc, xn, Nx, sF, sY, nullptr, sAr, L, LY, LO);
+    if (box_cell<T>(cl, i, j, x0, y0)) box_flux<T, false>(i, j, x0, y0, sF, sY, nullptr, L, LY, LO);
+    else group_flux<T, false>(Hx, Hy, sm_, x0, y0, xc, xn, Nx, sF, sY, nullptr, sAr, L, LY, LO);
     // axisymmetric hoop stress
     float r = fdiv(V, fmaxf(gg.y, 1e-6f)), vor = fdiv(vely, r);
     L.z -= T2h.x * (2.0f * vor - 0.6666667f * (T1h.x + T1h.w + vor)) * gg.y;
