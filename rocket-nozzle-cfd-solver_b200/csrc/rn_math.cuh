@@ -530,19 +530,34 @@ RN_DEV float rmix(float4 s, const rn_params& P) {
 }
 
 // FS_VCELL (solver.js:458-488) for one cell from its padded W/Wb and neighbours.
+// CENTRAL (fast variant): where all four neighbours are fluid, all but a few
+// cells along walls, the mean of the two one-sided differences is formed as the
+// central one.
+template <bool CENTRAL = false>
 RN_DEV void vcell(float4 w0, float4 sc, float4 wE, float4 wW, float4 wN, float4 wS, int i, int j, float l, float dt,
                   const rn_params& P, float4& T1, float4& T2) {
   T1 = make_float4(0.f, 0.f, 0.f, 0.f);
   T2 = T1;
   if (w0.x < 0.0f) return;
-  float fE = wE.x < 0.0f ? 0.0f : 1.0f, fW = wW.x < 0.0f ? 0.0f : 1.0f;
-  float fN = wN.x < 0.0f ? 0.0f : 1.0f, fS = wS.x < 0.0f ? 0.0f : 1.0f;
-  float dxn = fmaxf(fE + fW, 1.0f), drn = fmaxf(fN + fS, 1.0f);
-  const Over per_dx = over(dxn), per_dr = over(drn);
-  float ux = per_dx(fE * (wE.y - w0.y) + fW * (w0.y - wW.y));
-  float vx = per_dx(fE * (wE.z - w0.z) + fW * (w0.z - wW.z));
-  float ur = per_dr(fN * (wN.y - w0.y) + fS * (w0.y - wS.y));
-  float vr = per_dr(fN * (wN.z - w0.z) + fS * (w0.z - wS.z));
+  float ux, vx, ur, vr;
+#ifdef RN_FAST
+  if (CENTRAL && fminf(fminf(wE.x, wW.x), fminf(wN.x, wS.x)) > 0.0f) {
+    ux = 0.5f * (wE.y - wW.y);
+    vx = 0.5f * (wE.z - wW.z);
+    ur = 0.5f * (wN.y - wS.y);
+    vr = 0.5f * (wN.z - wS.z);
+  } else
+#endif
+  {
+    float fE = wE.x < 0.0f ? 0.0f : 1.0f, fW = wW.x < 0.0f ? 0.0f : 1.0f;
+    float fN = wN.x < 0.0f ? 0.0f : 1.0f, fS = wS.x < 0.0f ? 0.0f : 1.0f;
+    float dxn = fmaxf(fE + fW, 1.0f), drn = fmaxf(fN + fS, 1.0f);
+    const Over per_dx = over(dxn), per_dr = over(drn);
+    ux = per_dx(fE * (wE.y - w0.y) + fW * (w0.y - wW.y));
+    vx = per_dx(fE * (wE.z - w0.z) + fW * (w0.z - wW.z));
+    ur = per_dr(fN * (wN.y - w0.y) + fS * (w0.y - wS.y));
+    vr = per_dr(fN * (wN.z - w0.z) + fS * (w0.z - wS.z));
+  }
   float r = float(j) + 0.5f, vor = fdiv(w0.z, r);
   float div = ux + vr + vor;
   float S2 = 2.0f * (ux * ux + vr * vr + vor * vor) + (ur + vx) * (ur + vx) - 0.6666667f * div * div;

@@ -730,23 +730,60 @@ __device__ __forceinline__ void vcell_at(const Grid& g, const CellSrc<T>& cs, co
   }
   float4 T1 = make_float4(0.f, 0.f, 0.f, 0.f), T2 = T1;
   if (i >= 0 && i < Nx && j >= 0 && j < Nr)
-    vcell(sW[c], sWb[c], sW[c + 1], sW[c - 1], sW[c + rs], sW[c - rs], i, j,
+    vcell<!T::WIDE>(sW[c], sWb[c], sW[c + 1], sW[c - 1], sW[c + rs], sW[c - rs], i, j,
           (cs.cls(i, j) & CELL_L0) ? TURB_L0 : cs.gm(i, j).w, dt, P, T1, T2);
   sT1[k] = T1;
   sT2[k] = T2;
 }
 
-// FS_VFLUX_X/R: every viscous face of the tile and of its listed members in
-// one loop through one instance of the flux code (as the inviscid faces):
-// primitive slots p1 (behind the face) and p2 (the face's cell), vcell slots
-// v1 and v2; zero flux where it is not drawn or a side is a wall.
+// FS_VFLUX_X/R of face slot k, the face at (i, j): primitive slots p1 (behind
+// the face) and p2 (the face's cell), vcell slots v1 and v2; zero flux where it
+// is not drawn or a side is a wall.
+__device__ __forceinline__ void viscous_face(int k, bool dirR, int i, int j, int Nx, int Nr, int p1, int p2, int v1,
+                                             int v2, const float4* sW, const float4* sWb, const float4* sT1,
+                                             const float4* sT2, const float* sAr, float4* sF, float4* sY) {
+  const bool ok = dirR ? (i < Nx && j > 0 && j < Nr) : (i > 0 && i < Nx && j < Nr);
+  float4 F = make_float4(0.f, 0.f, 0.f, 0.f), FY = F;
+  if (ok) {
+    // face k is face k of the inviscid phase, whose open area sAr[k] holds
+    // (every face drawn here was drawn there)
+    const float area = sAr[k];
+    const float4 w1 = sW[p1], w2 = sW[p2];
+    if (area != 0.0f && !(w1.x < 0.0f || w2.x < 0.0f))
+      visc_flux(dirR, w1, sWb[p1], sT1[v1], sT2[v1], w2, sWb[p2], sT1[v2], sT2[v2], j, F, FY);
+  }
+  sF[k] = F;
+  sY[k] = FY;
+}
+// Tile x-face k or r-face k (row order within its direction).
+template <class T, bool DIR_R>
+__device__ __forceinline__ void viscous_tile_face(int k, const Grid& g, int x0, int y0, const float4* sW,
+                                                  const float4* sWb, const float4* sT1, const float4* sT2,
+                                                  const float* sAr, float4* sF, float4* sY) {
+  constexpr int W = DIR_R ? T::TX : T::TX + 1;
+  const int ly = k / W, lx = k - ly * W;
+  const int p2 = (ly + 2) * T::PX + lx + 2, v2 = (ly + 1) * T::TW + lx + 1;
+  viscous_face((DIR_R ? T::NXF : 0) + k, DIR_R, x0 + lx, y0 + ly, g.Nx, g.Nr, p2 - (DIR_R ? T::PX : 1), p2,
+               v2 - (DIR_R ? T::TW : 1), v2, sW, sWb, sT1, sT2, sAr, sF, sY);
+}
+// Every viscous face of the tile and of its listed members. WIDE shapes, and
+// those with more faces a direction than threads, run one flat list through one
+// instance of the flux code; the others a pass a direction with the direction
+// compiled in.
 template <class T>
 __device__ __forceinline__ void viscous_faces(const Grid& g, int x0, int y0, const int* xc, int xn, const float4* sW,
                                               const float4* sWb, const float4* sT1, const float4* sT2,
                                               const float* sAr, float4* sF, float4* sY) {
   constexpr int TX = T::TX, PX = T::PX, TW = T::TW, NXR = T::NXF + T::NRF;
-  const int Nx = g.Nx, Nr = g.Nr;
-  for (int k = threadIdx.x; k < NXR + 4 * xn; k += T::NT) {
+  constexpr bool PASSES = !T::WIDE && T::NXF <= T::NT && T::NRF <= T::NT;
+  const int Nx = g.Nx;
+  if constexpr (PASSES) {
+    for (int k = threadIdx.x; k < T::NXF; k += T::NT)
+      viscous_tile_face<T, false>(k, g, x0, y0, sW, sWb, sT1, sT2, sAr, sF, sY);
+    for (int k = threadIdx.x; k < T::NRF; k += T::NT)
+      viscous_tile_face<T, true>(k, g, x0, y0, sW, sWb, sT1, sT2, sAr, sF, sY);
+  }
+  for (int k = (PASSES ? NXR : 0) + threadIdx.x; k < NXR + 4 * xn; k += T::NT) {
     int i, j, p1, p2, v1, v2;
     bool dirR;
     if (k < NXR) {
@@ -767,18 +804,7 @@ __device__ __forceinline__ void viscous_faces(const Grid& g, int x0, int y0, con
       v1 = o ? vb : vb + (dirR ? 3 : 1);
       v2 = o ? vb + (dirR ? 4 : 2) : vb;
     }
-    const bool ok = dirR ? (i < Nx && j > 0 && j < Nr) : (i > 0 && i < Nx && j < Nr);
-    float4 F = make_float4(0.f, 0.f, 0.f, 0.f), FY = F;
-    if (ok) {
-      // face k is face k of the inviscid phase, whose open area sAr[k] holds
-      // (every face drawn here was drawn there)
-      const float area = sAr[k];
-      const float4 w1 = sW[p1], w2 = sW[p2];
-      if (area != 0.0f && !(w1.x < 0.0f || w2.x < 0.0f))
-        visc_flux(dirR, w1, sWb[p1], sT1[v1], sT2[v1], w2, sWb[p2], sT1[v2], sT2[v2], j, F, FY);
-    }
-    sF[k] = F;
-    sY[k] = FY;
+    viscous_face(k, dirR, i, j, Nx, g.Nr, p1, p2, v1, v2, sW, sWb, sT1, sT2, sAr, sF, sY);
   }
 }
 
