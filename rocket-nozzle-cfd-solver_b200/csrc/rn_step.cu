@@ -657,6 +657,15 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
   halo_issue<T>(a.tm, a.slotIn, x0, y0, RAW, sMask, bar);
   const FirstAreas fa = first_areas<T>(g, x0, y0);
   const CellSrc<T> cs{g, a.A, a.B, RAW, sMask, x0, y0, (x0 - 2) - ((x0 - 2) & ~15)};
+  // the step info with the member list's bounds, in one round of loads (the
+  // kernel before wrote it: dependent launches read it after their wait)
+  float4 info;
+  unsigned wmax;
+  const float4* const infoAt = STAGE == 1 ? a.stPrev : a.stNew;
+  if constexpr (!T::PDL) {
+    info = *infoAt;
+    if (STAGE == 1) wmax = *a.wIn;
+  }
   const int xb = a.xoff[tileId], xn = a.xoff[tileId + 1] - xb;
   const int NP = T::NPT + 25 * xn, NF = T::NXF + T::NRF + 4 * xn;
   float4* sF = R;
@@ -669,11 +678,15 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
   for (int q = NT - 1 - tid; q < xn; q += NT) xc[q] = a.xcell[xb + q];
 
   // from here on the block reads and writes what the kernel before it wrote or read
-  if constexpr (T::PDL) pdl_wait();
+  if constexpr (T::PDL) {
+    pdl_wait();
+    info = *infoAt;
+    if (STAGE == 1) wmax = *a.wIn;
+  }
   float dt, t;
   if (STAGE == 1) {
-    float4 prev = *a.stPrev;
-    float w = fmaxf(P.wFloor, __uint_as_float(*a.wIn));
+    const float4 prev = info;
+    float w = fmaxf(P.wFloor, __uint_as_float(wmax));
     dt = fminf(P.cfl / w, P.dtMax);
     if (prev.x > 0.0f) dt = fminf(dt, prev.x * 1.2f);
     t = prev.z;                                   // inlet ramp at t_old
@@ -682,9 +695,8 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
       *a.wOut = 0u;
     }
   } else {
-    float4 st = *a.stNew;
-    dt = st.x;
-    t = st.z;                                     // inlet ramp at t_new
+    dt = info.x;
+    t = info.z;                                   // inlet ramp at t_new
   }
   __syncthreads();
   if (!halo_wait(bar, a.err)) return;
@@ -990,6 +1002,8 @@ __device__ __forceinline__ void stage2_physics_body(const StageArgs& a, const Ph
   halo_issue<T>(a.tm, a.slotIn, x0, y0, RAW, sMask, bar);
   const FirstAreas fa = first_areas<T>(g, x0, y0);
   const CellSrc<T> cs{g, a.A, a.B, RAW, sMask, x0, y0, (x0 - 2) - ((x0 - 2) & ~15)};
+  float4 st;
+  if constexpr (!T::PDL) st = *a.stNew;           // with the member list's bounds, in one round of loads
   const int xb = a.xoff[tileId], xn = a.xoff[tileId + 1] - xb, xnP = P.visc ? xn : 0;
   const int NP = T::NPT + 25 * xn, NF = T::NXF + T::NRF + 4 * xn;
   const int NV = T::NTT + 5 * xnP;
@@ -1001,8 +1015,10 @@ __device__ __forceinline__ void stage2_physics_body(const StageArgs& a, const Ph
   float4* sW = reinterpret_cast<float4*>(sAr) + (NF + 3) / 4;
   float4* sWb = sW + NP;
   for (int q = NT - 1 - tid; q < xn; q += NT) xc[q] = a.xcell[xb + q];
-  if constexpr (T::PDL) pdl_wait();
-  const float4 st = *a.stNew;
+  if constexpr (T::PDL) {
+    pdl_wait();
+    st = *a.stNew;
+  }
   const float dt = st.x, t = st.z;
   __syncthreads();
   if (!halo_wait(bar, a.err)) return;
