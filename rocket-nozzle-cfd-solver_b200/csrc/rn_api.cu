@@ -77,8 +77,9 @@ void free_buffers(rn_solver* h) {
   h->liveSteps = nullptr;
   cudaFree(h->dHS);
   h->dHS = nullptr;
-  cudaFree(h->xoff); cudaFree(h->xcell); cudaFree(h->heavy);
-  h->xoff = h->xcell = nullptr;
+  cudaFree(h->xhead); cudaFree(h->xcell); cudaFree(h->heavy);
+  h->xhead = nullptr;
+  h->xcell = nullptr;
   h->heavy = nullptr;
   h->nHeavy = 0;
   cudaFree(h->mark); cudaFree(h->dRes); cudaFree(h->wallProf); cudaFree(h->derived);
@@ -354,12 +355,19 @@ int rn_build_member_lists(rn_solver* h) {
                                 std::to_string(MAXX) + ")");
   if (cells.empty()) cells.push_back(0);
   CK(cudaStreamSynchronize(h->stream));
-  cudaFree(h->xoff);
+  cudaFree(h->xhead);
   cudaFree(h->xcell);
-  h->xoff = h->xcell = nullptr;
-  CK(cudaMalloc(&h->xoff, sizeof(int) * (nT + 1)));
+  h->xhead = nullptr;
+  h->xcell = nullptr;
+  std::vector<MemberHead> head(nT);
+  for (int t = 0; t < nT; t++) {
+    head[t].first = off[t];
+    head[t].count = off[t + 1] - off[t];
+    for (int q = 0; q < HEAD_CELLS; q++) head[t].cell[q] = q < head[t].count ? cells[off[t] + q] : 0;
+  }
+  CK(cudaMalloc(&h->xhead, sizeof(MemberHead) * nT));
   CK(cudaMalloc(&h->xcell, sizeof(int) * cells.size()));
-  CK(cudaMemcpyAsync(h->xoff, off.data(), sizeof(int) * (nT + 1), cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemcpyAsync(h->xhead, head.data(), sizeof(MemberHead) * nT, cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->xcell, cells.data(), sizeof(int) * cells.size(), cudaMemcpyHostToDevice, h->stream));
   // tiles whose lists need more shared memory than the common launch holds
   std::vector<int> heavy;
@@ -647,7 +655,7 @@ int step_once(rn_solver* h, const rn_params* P) {
   a.oA = h->SA[s1]; a.oB = h->SB[s1];
   a.stPrev = stPrev; a.stNew = stNew; a.wIn = wIn; a.wOut = wOut;
   a.finalCfl = 0;
-  a.xoff = h->xoff; a.xcell = h->xcell; a.maxX = h->maxX;
+  a.xhead = h->xhead; a.xcell = h->xcell; a.maxX = h->maxX;
   a.slotIn = s0; a.tm = h->dMaps; a.err = h->errFlag;
   // The small shape's blocks leave room for the next kernel's, which set up
   // (barrier, mask, geometry, member lists) while this one runs: 320x120 16.7 ->
@@ -712,7 +720,6 @@ int step_once(rn_solver* h, const rn_params* P) {
     p.A1 = h->SA[s1]; p.B1 = h->SB[s1]; p.A2 = h->SA[s2]; p.B2 = h->SB[s2];
     p.oA = h->SA[s2]; p.oB = h->SB[s2];
     p.st = stNew; p.wOut = wOut; p.finalCfl = inj ? 0 : 1;
-    p.xoff = h->xoff; p.xcell = h->xcell; p.maxX = h->maxX;
     ProfScope ps(h, RN_K_STAGE2_PHYSICS);
     const int nTiles = int(h->hostXoff.size()) - 1;
     if (h->nHeavy > 0 && nTiles > SPLIT_BLOCKS_PER_SM * h->numSMs) {
@@ -773,7 +780,7 @@ int step_once(rn_solver* h, const rn_params* P) {
 // ring position the handle is at (up to one step of the two-step period).
 bool graph_matches(const rn_solver* h, const StepGraph& g, const rn_params* P) {
   return g.exec && g.K == h->K && g.tile == h->shape && g.maxX == h->maxX && g.nHeavy == h->nHeavy &&
-         g.base == h->SA[0] && g.xoff == h->xoff && std::memcmp(&g.P, P, sizeof(rn_params)) == 0;
+         g.base == h->SA[0] && g.xhead == h->xhead && std::memcmp(&g.P, P, sizeof(rn_params)) == 0;
 }
 bool graph_at_start(const rn_solver* h, const StepGraph& g, bool inj) {
   return h->cur == g.cur && h->stepIdx == g.stepIdx && h->wslot == g.wslot && (!inj || h->scur == g.scur);
@@ -839,7 +846,7 @@ int capture_steps(rn_solver* h, const rn_params* P, int B, StepGraph& g) {
   }
   if (gr) cudaGraphDestroy(gr);
   if (rc != RN_OK) return rc;
-  g.K = h->K; g.base = h->SA[0]; g.xoff = h->xoff;
+  g.K = h->K; g.base = h->SA[0]; g.xhead = h->xhead;
   g.tile = h->shape; g.maxX = h->maxX; g.nHeavy = h->nHeavy;
   g.cur = cur; g.stepIdx = stepIdx; g.wslot = wslot; g.scur = scur;
   g.steps = B;

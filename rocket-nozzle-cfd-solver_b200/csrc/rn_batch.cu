@@ -179,7 +179,7 @@ int refresh(rn_batch_t* b) {
     d.wmax = h->wmax;
     d.tm = h->dMaps;
     d.err = h->errFlag;
-    d.xoff = h->xoff;
+    d.xhead = h->xhead;
     d.xcell = h->xcell;
     normalise(b, h, d.cur0, d.stepIdx0, d.wslot0);
     d.firstBlock = first[m];

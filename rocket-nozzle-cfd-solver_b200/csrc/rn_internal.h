@@ -12,7 +12,7 @@
 // captured with (rn_step replays them only while all of that still holds).
 struct StepGraph {
   cudaGraphExec_t exec = nullptr;
-  const void *K = nullptr, *base = nullptr, *xoff = nullptr;
+  const void *K = nullptr, *base = nullptr, *xhead = nullptr;
   int tile = -1, maxX = -1, nHeavy = -1;
   int cur = -1, stepIdx = -1, wslot = -1, scur = -1;
   int steps = 0;
@@ -93,7 +93,7 @@ struct rn_solver {
   // They differ only while autoShape, i.e. until a caller sets the tile shape)
   int tile = RN_TILE_16x15, shape = RN_TILE_16x15;
   bool autoShape = true;
-  int* xoff = nullptr;
+  rn::MemberHead* xhead = nullptr;
   int* xcell = nullptr;
   int maxX = 1;
   std::vector<int> hostXoff;

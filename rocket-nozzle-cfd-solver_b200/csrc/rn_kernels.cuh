@@ -69,6 +69,15 @@ constexpr int XSMALL = 4;
 // 1024x384 grid (1,536 blocks) 3.67 -> 3.60, so it is not split.
 constexpr int SPLIT_BLOCKS_PER_SM = 16;
 
+// A tile's out-of-tile group members: how many, the first of them (most tiles
+// have fewer), and where the others are in the handle's cell list. One aligned
+// record, so that a block has its list after one round of loads.
+constexpr int HEAD_CELLS = 6;
+struct alignas(32) MemberHead {
+  int first, count;
+  int cell[HEAD_CELLS];
+};
+
 struct StageArgs {
   Grid g;
   const float4* A;  const float4* B;    // stage input state
@@ -79,8 +88,8 @@ struct StageArgs {
   const unsigned* wIn;                  // stage 1: max wave speed of the step's input state
   unsigned* wOut;                       // cleared by stage 1, accumulated by the step's last kernel
   int finalCfl;                         // this kernel writes the step's final state
-  const int* xoff;                      // per tile: out-of-tile members of its cut-cell groups (CSR)
-  const int* xcell;
+  const MemberHead* xhead;              // per tile: out-of-tile members of its cut-cell groups
+  const int* xcell;                     // all tiles' lists
   int maxX;                             // largest per-tile list (sizes the dynamic shared memory)
   int slotIn;                           // ring slot of (A, B): selects the tensor maps of the halo copy
   const TileMaps* tm;                   // the handle's tensor maps, one TileMaps per tile shape
@@ -96,9 +105,6 @@ struct PhysArgs {
   const float4* st;
   unsigned* wOut;
   int finalCfl;
-  const int* xoff;
-  const int* xcell;
-  int maxX;
 };
 
 struct SprayArgs {
@@ -141,7 +147,7 @@ struct BatchInst {
   float4* SB[3];
   float4* stepTex;                      // 2 float4
   unsigned* wmax;                       // 2 slots
-  const int* xoff;
+  const MemberHead* xhead;
   const int* xcell;
   const TileMaps* tm;                   // the member's tensor maps, one TileMaps per tile shape
   unsigned* err;                        // the member's error word (halo copy timeout)

@@ -84,7 +84,7 @@ size_t rn_handle_bytes(int Nx, int Nr) {
   b += sizeof(float4) * (2 + SPRAY_N * 7 + N + 768);   // step info, parcel ring + deposits, src, table
   b += sizeof(unsigned) * SPRAY_N * 4 + sizeof(double) * 16;
   b += rn::kernels_fast.sortTempBytes(int(N));
-  b += sizeof(int) * (N / 64 + 2) + sizeof(int) * 4096;  // member lists (generous)
+  b += sizeof(rn::MemberHead) * (N / 64 + 2) + sizeof(int) * 4096;  // member lists (generous)
   b += rn_residual_bytes(Nx, Nr);
   return (b + (1u << 20)) & ~size_t((1u << 20) - 1);   // allocation granularity slack
 }

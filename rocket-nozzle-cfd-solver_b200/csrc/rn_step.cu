@@ -9,7 +9,7 @@
 // and its 6 face textures never touch HBM here.
 //
 // Group members outside the tile (slivers merged across a tile edge) are
-// listed per tile at set_geometry (xoff/xcell). For each listed member the
+// listed per tile at set_geometry (xhead/xcell). For each listed member the
 // block adds a 5x5 block of primitives around it to the primitive phase and
 // its 4 faces to the face phase: the same loops and the same single instance
 // of the face code run them, so blocks along the walls do no serial or
@@ -59,6 +59,10 @@ struct TileT {
   static constexpr bool WIDE = WARPS_ < 32;
   // launched with programmatic dependence on the kernel before it (rn_api.cu)
   static constexpr bool PDL = ID_ == SHAPE_SMALL;
+  // the step info loaded with the member list's bounds, in one round: pays where
+  // a block's latency counts (viscous 512x192 21.6 -> 21.3 us), costs the
+  // 64-register shapes registers (plain 4096x1536 596 -> 609)
+  static constexpr bool EARLY_INFO = WIDE && !PDL;
   static constexpr int PX = TX + 4, PY = TY + 4, NPT = PX * PY;   // primitives with a 2-cell halo
   static constexpr int NXF = TY * (TX + 1), NRF = (TY + 1) * TX;  // x- and r-faces of a tile
   static constexpr int TW = TX + 2, NTT = (TX + 2) * (TY + 2);    // vcell ring (tile + 1)
@@ -657,16 +661,18 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
   halo_issue<T>(a.tm, a.slotIn, x0, y0, RAW, sMask, bar);
   const FirstAreas fa = first_areas<T>(g, x0, y0);
   const CellSrc<T> cs{g, a.A, a.B, RAW, sMask, x0, y0, (x0 - 2) - ((x0 - 2) & ~15)};
-  // the step info with the member list's bounds, in one round of loads (the
-  // kernel before wrote it: dependent launches read it after their wait)
+  // (the kernel before wrote the step info: dependent launches read it after
+  // their wait)
   float4 info;
   unsigned wmax;
   const float4* const infoAt = STAGE == 1 ? a.stPrev : a.stNew;
-  if constexpr (!T::PDL) {
+  if constexpr (T::EARLY_INFO) {
     info = *infoAt;
     if (STAGE == 1) wmax = *a.wIn;
   }
-  const int xb = a.xoff[tileId], xn = a.xoff[tileId + 1] - xb;
+  const MemberHead* const head = a.xhead + tileId;
+  const int xq = NT - 1 - tid;                   // member this thread lists (the first warp may wait for the kernel before)
+  const int xb = head->first, xn = head->count, xmine = xq < HEAD_CELLS ? head->cell[xq] : 0;
   const int NP = T::NPT + 25 * xn, NF = T::NXF + T::NRF + 4 * xn;
   float4* sF = R;
   float4* sY = sF + NF;
@@ -674,12 +680,11 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
   float* sAr = reinterpret_cast<float*>(R + stage_region_t<T>(xn));
   float4* sW = reinterpret_cast<float4*>(sAr) + (NF + 3) / 4;
   float4* sWb = sW + NP;
-  // (by the last threads: the first may wait for the kernel before)
-  for (int q = NT - 1 - tid; q < xn; q += NT) xc[q] = a.xcell[xb + q];
+  for (int q = xq; q < xn; q += NT) xc[q] = q < HEAD_CELLS ? xmine : a.xcell[xb + q];
 
   // from here on the block reads and writes what the kernel before it wrote or read
-  if constexpr (T::PDL) {
-    pdl_wait();
+  if constexpr (T::PDL) pdl_wait();
+  if constexpr (!T::EARLY_INFO) {
     info = *infoAt;
     if (STAGE == 1) wmax = *a.wIn;
   }
@@ -1003,8 +1008,10 @@ __device__ __forceinline__ void stage2_physics_body(const StageArgs& a, const Ph
   const FirstAreas fa = first_areas<T>(g, x0, y0);
   const CellSrc<T> cs{g, a.A, a.B, RAW, sMask, x0, y0, (x0 - 2) - ((x0 - 2) & ~15)};
   float4 st;
-  if constexpr (!T::PDL) st = *a.stNew;           // with the member list's bounds, in one round of loads
-  const int xb = a.xoff[tileId], xn = a.xoff[tileId + 1] - xb, xnP = P.visc ? xn : 0;
+  if constexpr (T::EARLY_INFO) st = *a.stNew;
+  const MemberHead* const head = a.xhead + tileId;
+  const int xq = NT - 1 - tid;                   // member this thread lists
+  const int xb = head->first, xn = head->count, xnP = P.visc ? xn : 0, xmine = xq < HEAD_CELLS ? head->cell[xq] : 0;
   const int NP = T::NPT + 25 * xn, NF = T::NXF + T::NRF + 4 * xn;
   const int NV = T::NTT + 5 * xnP;
   float4* sT1 = T::WIDE ? R + fused_region8_t<T>(xn) : R;
@@ -1014,11 +1021,9 @@ __device__ __forceinline__ void stage2_physics_body(const StageArgs& a, const Ph
   float* sAr = reinterpret_cast<float*>(sB2 + T::NC + xn);   // face areas, kept for FS_SOURCE
   float4* sW = reinterpret_cast<float4*>(sAr) + (NF + 3) / 4;
   float4* sWb = sW + NP;
-  for (int q = NT - 1 - tid; q < xn; q += NT) xc[q] = a.xcell[xb + q];
-  if constexpr (T::PDL) {
-    pdl_wait();
-    st = *a.stNew;
-  }
+  for (int q = xq; q < xn; q += NT) xc[q] = q < HEAD_CELLS ? xmine : a.xcell[xb + q];
+  if constexpr (T::PDL) pdl_wait();
+  if constexpr (!T::EARLY_INFO) st = *a.stNew;
   const float dt = st.x, t = st.z;
   __syncthreads();
   if (!halo_wait(bar, a.err)) return;
@@ -1132,7 +1137,7 @@ __global__ void __launch_bounds__(T::NT, T::MINB) k_stage2phys(StageArgs a, Phys
     bx = blockIdx.x;
     by = blockIdx.y;
     tile = by * gridDim.x + bx;
-    if (xSmall >= 0 && a.xoff[tile + 1] - a.xoff[tile] > xSmall) return;
+    if (xSmall >= 0 && a.xhead[tile].count > xSmall) return;
   }
   stage2_physics_body<T>(a, p, P, bx, by, tile, sm, red, xc, &bar);
 }
@@ -1169,7 +1174,7 @@ __device__ __forceinline__ void batch_stage_args(const BatchInst& d, const Batch
   a.wIn = d.wmax + ws;
   a.wOut = d.wmax + (1 - ws);
   a.finalCfl = ph.finalCfl;
-  a.xoff = d.xoff; a.xcell = d.xcell; a.maxX = ph.maxX;
+  a.xhead = d.xhead; a.xcell = d.xcell; a.maxX = ph.maxX;
   a.slotIn = stage == 1 ? s0 : s1;
   a.tm = d.tm;
   a.err = d.err;
@@ -1205,7 +1210,7 @@ __global__ void __launch_bounds__(T::NT, T::MINB) k_stage2phys_batch(const Batch
   if (ph.active && !ph.active[inst]) return;      // a member stopped by rn_batch_run: the whole block
   load_inst(insts, inst, d);
   const int local = heavy ? hv.y : blockIdx.x - d.firstBlock, by = local / d.tilesX, bx = local - by * d.tilesX;
-  if (!heavy && xSmall >= 0 && d.xoff[local + 1] - d.xoff[local] > xSmall) return;   // in the heavy launch
+  if (!heavy && xSmall >= 0 && d.xhead[local].count > xSmall) return;   // in the heavy launch
   if (threadIdx.x == 0) {
     batch_stage_args(d, ph, 2, a);
     a.finalCfl = 0;
@@ -1217,7 +1222,6 @@ __global__ void __launch_bounds__(T::NT, T::MINB) k_stage2phys_batch(const Batch
     p.st = d.stepTex + (1 - si);
     p.wOut = d.wmax + (1 - ws);
     p.finalCfl = ph.finalCfl;
-    p.xoff = d.xoff; p.xcell = d.xcell; p.maxX = ph.maxX;
   }
   __syncthreads();
   stage2_physics_body<T>(a, p, insts[inst].P, bx, by, local, sm, red, xc, &bar);
