@@ -657,13 +657,20 @@ int step_once(rn_solver* h, const rn_params* P) {
   a.finalCfl = 0;
   a.xhead = h->xhead; a.xcell = h->xcell; a.maxX = h->maxX;
   a.slotIn = s0; a.tm = h->dMaps; a.err = h->errFlag;
-  // The small shape's blocks leave room for the next kernel's, which set up
-  // (barrier, mask, geometry, member lists) while this one runs: 320x120 16.7 ->
-  // 15.8 us a viscous step, 12.3 -> 11.3 an inviscid one. Not for the larger
-  // shapes: as slots come free one by one, consecutive blocks, the costly ones
-  // of a wall among them, gather on one SM (14x16, viscous 512x192: 21.9 ->
-  // 23.2 us).
-  a.pdl = !inj && !h->prof && h->shape == SHAPE_SMALL;
+  // Dependent launches: the next kernel's blocks set up (barrier, mask,
+  // geometry, member lists) while this one runs. The small shape's blocks leave
+  // room for them: 320x120 16.7 -> 15.8 us a viscous step, 12.3 -> 11.3 an
+  // inviscid one. 14x16 blocks at two to three an SM: they come as slots free,
+  // three an SM in the end as without (512x192: inviscid 16.1 -> 14.7 us); the
+  // fused kernel is launched after its predecessor all the same, since blocks
+  // that come in that order gather the costly wall tiles on an SM (viscous 21.5
+  // -> 21.0 us so, 23.2 with both kernels dependent). With two blocks an SM or
+  // fewer, early blocks would make three on some (400x150: 14.0 -> 14.7 us).
+  {
+    const int tiles = tile_count(h->shape, h->Nx, h->Nr);
+    a.pdl = !inj && !h->prof &&
+            (h->shape == SHAPE_SMALL || (h->shape == RN_TILE_14x16 && tiles > 2 * h->numSMs && tiles <= 3 * h->numSMs));
+  }
   {
     ProfScope ps(h, RN_K_STAGE1);
     h->K->stage1(a, *P, h->shape, h->stream);

@@ -57,11 +57,13 @@ struct TileT {
   // memory, loop body and live registers cost more than they save (64 batched
   // instances, 16x15: 4.37 -> 4.18 G).
   static constexpr bool WIDE = WARPS_ < 32;
-  // launched with programmatic dependence on the kernel before it (rn_api.cu)
-  static constexpr bool PDL = ID_ == SHAPE_SMALL;
-  // the step info loaded with the member list's bounds, in one round: pays where
-  // a block's latency counts (viscous 512x192 21.6 -> 21.3 us), costs the
-  // 64-register shapes registers (plain 4096x1536 596 -> 609)
+  // kernels that may be launched with programmatic dependence on the one before
+  // (rn_api.cu): all of the small shape's, 14x16's stage kernels
+  static constexpr bool PDL = ID_ == SHAPE_SMALL, PDL_STAGE = PDL || ID_ == 4;
+  // the fused kernel's step info loaded with the member list's bounds, in one
+  // round: pays where a block's latency counts and it need not wait for the
+  // kernel before (viscous 512x192 21.6 -> 21.3 us), costs the 64-register
+  // shapes registers
   static constexpr bool EARLY_INFO = WIDE && !PDL;
   static constexpr int PX = TX + 4, PY = TY + 4, NPT = PX * PY;   // primitives with a 2-cell halo
   static constexpr int NXF = TY * (TX + 1), NRF = (TY + 1) * TX;  // x- and r-faces of a tile
@@ -212,19 +214,19 @@ __device__ __forceinline__ float member_face_area(const Grid& g, int q, const in
 // mbarrier and issues its tiled copies: the state of the tile + 2-cell halo
 // (raw A into R, raw B into R + NPT8), the mask block (its box starts at the
 // 16-byte boundary at or below the halo's first column) and, for WIDE shapes,
-// the geometry boxes. With dependent launches (PDL) the mask and geometry,
+// the geometry boxes. Where launches may be dependent (PDL) the mask and geometry,
 // which no kernel of the step writes, go first, then, after the kernel before,
 // the state it wrote. The other threads meanwhile load face areas and the
 // member list.
-template <class T>
+template <class T, bool PDL>
 __device__ __forceinline__ void halo_issue(const TileMaps* tm, int slot, int x0, int y0, float4* R, uint8_t* sMask,
                                            uint64_t* bar) {
-  if constexpr (T::PDL) pdl_launch();
+  pdl_launch();
   if (threadIdx.x == 0) {
     const TileMaps& M = tm[T::ID];
     mbar_init(bar, 1);
     mbar_expect_tx(bar, T::HALO_BYTES + (T::WIDE ? T::GEO_BYTES : 0u));
-    if constexpr (!T::PDL) {
+    if constexpr (!PDL) {
       tma_load_2d(R, &M.a[slot], 4 * (x0 - 2), y0 - 2, bar);
       tma_load_2d(R + T::NPT8, &M.b[slot], 4 * (x0 - 2), y0 - 2, bar);
     }
@@ -233,7 +235,7 @@ __device__ __forceinline__ void halo_issue(const TileMaps* tm, int slot, int x0,
       tma_load_2d(R + 2 * T::NPT8, &M.geoM, 4 * (x0 - 1), y0 - 1, bar);
       tma_load_2d(R + 2 * T::NPT8 + T::NGM8, &M.geoG, 4 * x0, y0, bar);
     }
-    if constexpr (T::PDL) {
+    if constexpr (PDL) {
       pdl_wait();
       tma_load_2d(R, &M.a[slot], 4 * (x0 - 2), y0 - 2, bar);
       tma_load_2d(R + T::NPT8, &M.b[slot], 4 * (x0 - 2), y0 - 2, bar);
@@ -658,18 +660,9 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
   uint8_t* sMask = reinterpret_cast<uint8_t*>(sm);
   float4* RAW = sm + T::MASKF4;                 // raw halo block (+ geometry boxes for WIDE shapes)
   float4* R = RAW + T::STAGED_F4;               // face fluxes (other shapes: over the raw block)
-  halo_issue<T>(a.tm, a.slotIn, x0, y0, RAW, sMask, bar);
+  halo_issue<T, T::PDL_STAGE>(a.tm, a.slotIn, x0, y0, RAW, sMask, bar);
   const FirstAreas fa = first_areas<T>(g, x0, y0);
   const CellSrc<T> cs{g, a.A, a.B, RAW, sMask, x0, y0, (x0 - 2) - ((x0 - 2) & ~15)};
-  // (the kernel before wrote the step info: dependent launches read it after
-  // their wait)
-  float4 info;
-  unsigned wmax;
-  const float4* const infoAt = STAGE == 1 ? a.stPrev : a.stNew;
-  if constexpr (T::EARLY_INFO) {
-    info = *infoAt;
-    if (STAGE == 1) wmax = *a.wIn;
-  }
   const MemberHead* const head = a.xhead + tileId;
   const int xq = NT - 1 - tid;                   // member this thread lists (the first warp may wait for the kernel before)
   const int xb = head->first, xn = head->count, xmine = xq < HEAD_CELLS ? head->cell[xq] : 0;
@@ -683,15 +676,11 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
   for (int q = xq; q < xn; q += NT) xc[q] = q < HEAD_CELLS ? xmine : a.xcell[xb + q];
 
   // from here on the block reads and writes what the kernel before it wrote or read
-  if constexpr (T::PDL) pdl_wait();
-  if constexpr (!T::EARLY_INFO) {
-    info = *infoAt;
-    if (STAGE == 1) wmax = *a.wIn;
-  }
+  if constexpr (T::PDL_STAGE) pdl_wait();
   float dt, t;
   if (STAGE == 1) {
-    const float4 prev = info;
-    float w = fmaxf(P.wFloor, __uint_as_float(wmax));
+    float4 prev = *a.stPrev;
+    float w = fmaxf(P.wFloor, __uint_as_float(*a.wIn));
     dt = fminf(P.cfl / w, P.dtMax);
     if (prev.x > 0.0f) dt = fminf(dt, prev.x * 1.2f);
     t = prev.z;                                   // inlet ramp at t_old
@@ -700,8 +689,9 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
       *a.wOut = 0u;
     }
   } else {
-    dt = info.x;
-    t = info.z;                                   // inlet ramp at t_new
+    float4 st = *a.stNew;
+    dt = st.x;
+    t = st.z;                                     // inlet ramp at t_new
   }
   __syncthreads();
   if (!halo_wait(bar, a.err)) return;
@@ -1004,7 +994,7 @@ __device__ __forceinline__ void stage2_physics_body(const StageArgs& a, const Ph
   uint8_t* sMask = reinterpret_cast<uint8_t*>(sm);
   float4* RAW = sm + T::MASKF4;                 // raw halo block (+ geometry boxes for WIDE shapes)
   float4* R = RAW + T::STAGED_F4;               // face region (other shapes: over the raw block)
-  halo_issue<T>(a.tm, a.slotIn, x0, y0, RAW, sMask, bar);
+  halo_issue<T, T::PDL>(a.tm, a.slotIn, x0, y0, RAW, sMask, bar);
   const FirstAreas fa = first_areas<T>(g, x0, y0);
   const CellSrc<T> cs{g, a.A, a.B, RAW, sMask, x0, y0, (x0 - 2) - ((x0 - 2) & ~15)};
   float4 st;
@@ -1429,7 +1419,7 @@ static void stage2phys_t(const StageArgs& a, const PhysArgs& p, const rn_params&
     const int xs = a.maxX < XSMALL ? a.maxX : XSMALL;
     launch_step(k_stage2phys<T>, tiles_of<T>(a.g), T::NT, fused_smem_t<T>(xs), s, false, a, p, P, none, XSMALL);
   } else {
-    launch_step(k_stage2phys<T>, tiles_of<T>(a.g), T::NT, fused_smem_t<T>(a.maxX), s, a.pdl != 0, a, p, P, none, -1);
+    launch_step(k_stage2phys<T>, tiles_of<T>(a.g), T::NT, fused_smem_t<T>(a.maxX), s, a.pdl != 0 && T::PDL, a, p, P, none, -1);
   }
 }
 void launch_stage2phys(const StageArgs& a, const PhysArgs& p, const rn_params& P, int tile, const int* heavy,
