@@ -256,26 +256,28 @@ int rn_build_tile_maps(rn_solver* h) {
 }
 
 __global__ void k_cell_classes(Grid g, uint8_t* __restrict__ out, int pitch) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
-  if (i >= g.Nx) return;
-  const int k = j * g.Nx + i;
-  const float4 gm = g.geoM[k], gg = g.geoG[k], ga = g.geoA[j * (g.Nx + 1) + i];
-  const int z = __float2int_rn(gm.z);
-  const float row = float(j);
-  int c = g.mask[k] ? CELL_SOLID : 0;
-  if (!c && gm.x == 0.0f && gm.y == 0.0f && (z & 15) == 0 && gg.x == row + 0.5f && gg.y == 1.0f && gg.z == 0.0f &&
-      gg.w == 0.0f)
-    c |= CELL_PLAIN;
-  if (!(z & 16)) c |= CELL_NO_BAND;
-  if (gm.w == TURB_L0) c |= CELL_L0;
-  if (ga.z == row + 0.5f && ga.w == row) c |= CELL_FACES;
-  const float east = g.geoA[j * (g.Nx + 1) + i + 1].z, north = g.geoA[(j + 1) * (g.Nx + 1) + i].w;
-  if (fabsf(ga.z) == row + 0.5f && fabsf(ga.w) == row && fabsf(east) == row + 0.5f && fabsf(north) == row + 1.0f)
-    c |= CELL_BOX;
-  out[size_t(j) * pitch + i] = uint8_t(c);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int j = blockIdx.y; j < g.Nr && i < g.Nx; j += gridDim.y) {
+    const int k = j * g.Nx + i;
+    const float4* const fa = g.geoA + (size_t(j) * (g.Nx + 1) + i);
+    const float4 gm = g.geoM[k], gg = g.geoG[k], ga = fa[0];
+    const float east = fa[1].z, north = fa[g.Nx + 1].w;
+    const int z = __float2int_rn(gm.z);
+    const float row = float(j);
+    int c = g.mask[k] ? CELL_SOLID : 0;
+    if (!c && gm.x == 0.0f && gm.y == 0.0f && (z & 15) == 0 && gg.x == row + 0.5f && gg.y == 1.0f && gg.z == 0.0f &&
+        gg.w == 0.0f)
+      c |= CELL_PLAIN;
+    if (!(z & 16)) c |= CELL_NO_BAND;
+    if (gm.w == TURB_L0) c |= CELL_L0;
+    if (ga.z == row + 0.5f && ga.w == row) c |= CELL_FACES;
+    if (fabsf(ga.z) == row + 0.5f && fabsf(ga.w) == row && fabsf(east) == row + 0.5f && fabsf(north) == row + 1.0f)
+      c |= CELL_BOX;
+    out[size_t(j) * pitch + i] = uint8_t(c);
+  }
 }
 int rn_classes_refresh(rn_solver* h) {
-  k_cell_classes<<<dim3((h->Nx + 127) / 128, h->Nr), 128, 0, h->stream>>>(h->grid(), h->maskP, h->maskPitch);
+  k_cell_classes<<<dim3((h->Nx + 127) / 128, std::min(h->Nr, 65535)), 128, 0, h->stream>>>(h->grid(), h->maskP, h->maskPitch);
   CK(cudaGetLastError());
   return RN_OK;
 }
@@ -668,7 +670,7 @@ int step_once(rn_solver* h, const rn_params* P) {
   // fewer, early blocks would make three on some (400x150: 14.0 -> 14.7 us).
   {
     const int tiles = tile_count(h->shape, h->Nx, h->Nr);
-    a.pdl = !inj && !h->prof &&
+    a.pdl = !h->prof &&
             (h->shape == SHAPE_SMALL || (h->shape == RN_TILE_14x16 && tiles > 2 * h->numSMs && tiles <= 3 * h->numSMs));
   }
   {
@@ -682,6 +684,7 @@ int step_once(rn_solver* h, const rn_params* P) {
     sp.A1 = h->SA[s1]; sp.B1 = h->SB[s1];
     sp.PA = h->PA[h->scur]; sp.PB = h->PB[h->scur];
     sp.oPA = h->PA[1 - h->scur]; sp.oPB = h->PB[1 - h->scur]; sp.oPC = h->PC[1 - h->scur];
+    sp.cls = h->maskP; sp.clsPitch = h->maskPitch;
     sp.tab = h->tab; sp.st = stNew;
     sp.key = h->key; sp.val = h->val; sp.dep = h->dep;
     sp.acc = h->acc + size_t(4) * g.Nx * g.Nr * h->scur;
@@ -719,6 +722,7 @@ int step_once(rn_solver* h, const rn_params* P) {
   b.A = h->SA[s1]; b.B = h->SB[s1]; b.A0 = h->SA[s0]; b.B0 = h->SB[s0];
   b.oA = h->SA[s2]; b.oB = h->SB[s2];
   b.slotIn = s1;
+  if (inj) b.pdl = 0;                         // the parcel step forks off between the two kernels
   b.finalCfl = (!phys && !inj) ? 1 : 0;
   if (phys) {
     // stage 2 + split step in one kernel; its output replaces the stage-2 slot
@@ -758,6 +762,7 @@ int step_once(rn_solver* h, const rn_params* P) {
     ApplyArgs ap;
     ap.g = g;
     ap.A = h->SA[h->cur]; ap.B = h->SB[h->cur]; ap.src = h->src;
+    ap.cls = h->maskP; ap.clsPitch = h->maskPitch;
     ap.acc = h->acc + size_t(4) * g.Nx * g.Nr * h->scur;
     ap.accNext = h->acc + size_t(4) * g.Nx * g.Nr * (1 - h->scur);
     ap.boundIn = h->depBound + 2 * h->scur;

@@ -281,6 +281,7 @@ int launch_step(rn_batch_t* b, int c, bool withSpray) {
       sp.A1 = h->SA[s1]; sp.B1 = h->SB[s1];
       sp.PA = h->PA[h->scur]; sp.PB = h->PB[h->scur];
       sp.oPA = h->PA[1 - h->scur]; sp.oPB = h->PB[1 - h->scur]; sp.oPC = h->PC[1 - h->scur];
+      sp.cls = h->maskP; sp.clsPitch = h->maskPitch;
       sp.tab = h->tab; sp.st = h->stepTex + (1 - si);
       sp.key = h->key; sp.val = h->val; sp.dep = h->dep;
       sp.acc = h->acc + size_t(4) * h->Nx * h->Nr * h->scur;
@@ -329,6 +330,7 @@ int launch_step(rn_batch_t* b, int c, bool withSpray) {
       ApplyArgs ap;
       ap.g = h->grid();
       ap.A = h->SA[cur]; ap.B = h->SB[cur]; ap.src = h->src;
+      ap.cls = h->maskP; ap.clsPitch = h->maskPitch;
       ap.acc = h->acc + size_t(4) * h->Nx * h->Nr * h->scur;
       ap.accNext = h->acc + size_t(4) * h->Nx * h->Nr * (1 - h->scur);
       ap.boundIn = h->depBound + 2 * h->scur;

@@ -112,6 +112,8 @@ struct SprayArgs {
   const float4* A1; const float4* B1;   // stage-1 state: the gas the parcels see
   const float4* PA; const float4* PB;   // parcels before the step
   float4* oPA; float4* oPB; float4* oPC;
+  const uint8_t* cls;                   // cell classes, rows of clsPitch bytes
+  int clsPitch;
   const float4* tab;                    // 256 x 3 injector table
   const float4* st;
   unsigned* key; unsigned* val; float4* dep;   // deposit records (cell key, parcel index, source)
@@ -128,6 +130,8 @@ struct ApplyArgs {
   Grid g;
   const float4* A; const float4* B;
   const float4* src;
+  const uint8_t* cls;                   // cell classes, rows of clsPitch bytes
+  int clsPitch;
   const unsigned long long* acc;        // this step's fixed-point deposit sums (fast variant)
   const unsigned* boundIn;              // the (mass, speed) bounds its deposits were scaled by
   unsigned long long* accNext;          // the next step's, cleared here cell by cell

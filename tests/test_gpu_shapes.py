@@ -103,3 +103,36 @@ def test_cell_classes_follow_the_geometry(rn, oracle, kind, tile):
         assert max(state_rel_l2(a, o.readAll()).values()) <= 1e-6
     g.close()
     ref.close()
+
+
+@pytest.mark.parametrize("Nx,Nr", [(128, 48), (300, 61), (512, 130)])
+def test_spray_steps_on_each_default_shape(rn, oracle, Nx, Nr):
+    """Spray steps (the parcel step and the apply by cell classes, dependent
+    launches after the apply) against the oracle in exact precision, through
+    single launches and graph replays, on grids of the small shape and of 14x16
+    with up to two and up to three blocks an SM. Bar of the exact precision's
+    spray cases: only pow, exp, log, sin and cos may differ, in the last bit."""
+    from helpers import state_rel_l2
+    from rocket_nozzle_cfd_solver_b200 import configs
+    s = rn.build_sim_setup(configs.injector_spray(Nx, Nr)[0])
+    PA, PB, head = configs.prepopulated_parcels(s, 5000)
+    init = s.initialState()
+    g = rn.GPUSolver(Nx, Nr)
+    g.setPrecision("exact")
+    g.setGeometry(s.geo)
+    g.setState(init["A"], init["B"])
+    rn.GPUSpray(g).resize()
+    g.spray.setInjector(s.injector)
+    g.spray.setParcels(PA, PB, head)
+    o = oracle.OracleSolver(Nx, Nr)
+    o.setGeometry(s.geo)
+    o.setState(init["A"], init["B"])
+    o.setInjector(s.injector)
+    o.setParcels(PA, PB, head)
+    for n in (1, 2, 9, 8):
+        g.step(n, s.P)
+        o.step(n, s.P)
+    assert max(state_rel_l2(g.readAll(), o.readAll()).values()) <= 1e-5
+    alive = lambda p: np.asarray(p).reshape(-1, 4)[:, 1] > 0  # noqa: E731
+    assert np.array_equal(alive(g.spray.readParcels()["PB"]), alive(o.readParcels()["PB"]))
+    g.close()
