@@ -99,17 +99,18 @@ static_assert(4 * Tile3::PX <= 256 && Tile3::MW <= 256 && Tile0::PY <= 256, "cop
 constexpr unsigned HALO_WAIT_POLLS = 1u << 22;
 
 // --------------------------------------------------------------------------
-// block-wide max of non-negative floats -> one atomicMax on the bit pattern
+// block-wide max of non-negative floats (NaN counts as 0) -> one atomicMax on the
+// bit pattern, whose order is the floats': a warp's max is one reduction
+// instruction where shuffles take five dependent steps
 template <int NT>
 __device__ __forceinline__ void block_max_to(float w, unsigned* out, float* red) {
-  for (int o = 16; o > 0; o >>= 1) w = fmaxf(w, __shfl_xor_sync(0xffffffffu, w, o));
+  unsigned u = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(w, 0.0f)));
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) red[wid] = w;
+  if (lane == 0) red[wid] = __uint_as_float(u);
   __syncthreads();
   if (wid == 0) {
-    w = lane < (NT / 32) ? red[lane] : 0.0f;
-    for (int o = 16; o > 0; o >>= 1) w = fmaxf(w, __shfl_xor_sync(0xffffffffu, w, o));
-    if (lane == 0 && w > 0.0f) atomicMax(out, __float_as_uint(w));
+    u = __reduce_max_sync(0xffffffffu, lane < (NT / 32) ? __float_as_uint(red[lane]) : 0u);
+    if (lane == 0 && u != 0u) atomicMax(out, u);
   }
 }
 
@@ -288,10 +289,12 @@ struct CellSrc {
   }
 };
 // Every thread waits for the halo copy (after a barrier that published the
-// mbarrier's initialisation). False, in every thread, when any thread gave
-// up; the block then records the error and leaves.
-__device__ __forceinline__ bool halo_wait(uint64_t* bar, unsigned* err) {
-  const bool ok = mbar_wait_bounded(bar, HALO_WAIT_POLLS);
+// mbarrier's initialisation); false when it gave up. The block goes on to the
+// primitives either way (they only read what the copies left in shared memory)
+// and leaves together at the barrier after them (halo_ok), where any thread that
+// gave up makes it record the error: no barrier of the wait's own.
+__device__ __forceinline__ bool halo_wait(uint64_t* bar) { return mbar_wait_bounded(bar, HALO_WAIT_POLLS); }
+__device__ __forceinline__ bool halo_ok(bool ok, unsigned* err) {
   if (__syncthreads_and(ok)) return true;
   if (threadIdx.x == 0 && err) atomicOr(err, 1u);
   return false;
@@ -694,10 +697,10 @@ __device__ __forceinline__ void stage_body(const StageArgs& a, const rn_params& 
     t = st.z;                                     // inlet ramp at t_new
   }
   __syncthreads();
-  if (!halo_wait(bar, a.err)) return;
+  const bool arrived = halo_wait(bar);
   load_prims<T>(g, a.A, a.B, t, P, x0, y0, xc, NP, RAW, sMask, sW, sWb);
   store_areas<T>(g, x0, y0, xc, xn, fa, sMask, sAr);
-  __syncthreads();
+  if (!halo_ok(arrived, a.err)) return;
   inviscid_faces<T>(P, xn, sW, sWb, sF, sY, sO, sAr);
   __syncthreads();
 
@@ -1016,10 +1019,10 @@ __device__ __forceinline__ void stage2_physics_body(const StageArgs& a, const Ph
   if constexpr (!T::EARLY_INFO) st = *a.stNew;
   const float dt = st.x, t = st.z;
   __syncthreads();
-  if (!halo_wait(bar, a.err)) return;
+  const bool arrived = halo_wait(bar);
   load_prims<T>(g, a.A, a.B, t, P, x0, y0, xc, NP, RAW, sMask, sW, sWb);
   store_areas<T>(g, x0, y0, xc, xn, fa, sMask, sAr);
-  __syncthreads();
+  if (!halo_ok(arrived, a.err)) return;
   {
     float4* sF = R;
     float4* sY = sF + NF;
