@@ -199,10 +199,12 @@ int rn_get_precision(rn_handle h, int* mode);
 /* Tile shape of the stage/physics kernels (a thread per cell):
  * RN_TILE_16x15, RN_TILE_16x16, RN_TILE_16x8, RN_TILE_32x15 or RN_TILE_14x16. A new handle
  * starts with RN_TILE_14x16 when the grid's 14 x 16 tiles number at most 3 per
- * SM (all resident at once), else with RN_TILE_16x15. rn_autotune times `steps` steps
- * with each shape on a copy of the handle's current state (the state, step
- * info and spray ring are restored afterwards), keeps the fastest and returns
- * it in *chosen. No reference counterpart (the reference draws full-screen
+ * SM (all resident at once), else with RN_TILE_16x15; until a shape is set its
+ * kernels may run another that suits the grid's size better (10 x 10 on small
+ * grids, 16 x 16 where it divides the height better) under that name.
+ * rn_autotune times `steps` steps with each shape, that one included, on a copy
+ * of the handle's current state (the state, step info and spray ring are
+ * restored afterwards), keeps the fastest and returns its name in *chosen. No reference counterpart (the reference draws full-screen
  * fragment passes). */
 #define RN_TILE_16x16 0
 #define RN_TILE_16x8 1
@@ -246,7 +248,8 @@ int rn_batch_step(rn_batch b, int n);
  * frame loop (app.js:965 calls step(n, P) until the user stops it). */
 int rn_batch_run(rn_batch b, const double* t_end, int chunk, long long max_steps, long long* steps);
 int rn_batch_sync(rn_batch b);
-/* tile shape of the batch's launches (RN_TILE_*) */
+/* tile shape of the batch's launches (RN_TILE_*); RN_TILE_16x15 until set, run
+ * as 16 x 16 where the members' grids need clearly fewer tiles of that */
 int rn_batch_set_tile(rn_batch b, int shape);
 /* times `steps` batch steps with each tile shape on copies of the members'
  * current states (states, step info and spray rings are restored), keeps the

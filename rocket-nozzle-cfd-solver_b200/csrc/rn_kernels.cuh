@@ -36,10 +36,10 @@ inline int tile_count(int shape, int Nx, int Nr) {
   return ((Nx + TILE_TX[shape] - 1) / TILE_TX[shape]) * ((Nr + TILE_TY[shape] - 1) / TILE_TY[shape]);
 }
 // 16x16 in place of 16x15 where it needs clearly fewer tiles for the same grids
-// (heights that 15 divides badly): a 16x16 tile costs about 7 % more. us per
-// step, 16x15 / 16x16: viscous 1024x287 (1280 / 1152 tiles) 54.2 / 50.8, 64
-// batched 128x48 (2048 / 1536) 108 / 97; 1024x384 (1664 / 1536) 67.8 / 72.3, 24
-// batched mixed grids (2224 / 2040 a set of four) 622 / 694.
+// (heights that 15 divides badly): a 16x16 tile costs more than its 7 % of cells.
+// us per step, 16x15 / 16x16: viscous 1024x287 (1280 / 1152 tiles) 48.9 / 45.7,
+// 64 batched 128x48 (2048 / 1536) 103 / 92; 1024x384 (1664 / 1536) 59.1 / 65.8, 24
+// batched mixed grids (2224 / 2040 a set of four) 540 / 602.
 inline bool prefer_16x16(long long tiles16x16, long long tiles16x15) { return 11 * tiles16x16 <= 10 * tiles16x15; }
 // A cell's class byte, in the row-pitched plane that the step kernels copy with
 // the halo (0 outside the grid). Almost all cells are uncut (99 % of the plume
