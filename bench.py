@@ -38,9 +38,19 @@ FLUSH_BYTES = 512 << 20     # > 126 MB L2
 WORKLOAD = "viscous plume 512x192 (methalox gamma 1.2, T0 3500 K, p0 70 bar, bell eps 20, sea level)"
 # algorithmic HBM bytes per cell for each kernel kind (fused design): state
 # planes are 32 B per cell (A 16 + B 16), geometry 49 B (geoA, geoG, geoM 16
-# each + mask 1); spray parcels 112 B each.
-BYTES_PER_CELL = {"stage1": 32 + 49 + 32, "stage2": 32 + 32 + 49 + 32, "stage2_physics": 32 + 32 + 49 + 32,
-                  "apply": 32 + 16 + 33 + 32, "reduce": 32 + 1}
+# each + the class byte) in the 14x16 kernels, the class byte alone in the other
+# shapes (uncut cells' geometry is formed, not read); spray parcels 112 B each.
+STATE_BYTES = {"stage1": 32 + 32, "stage2": 32 + 32 + 32, "stage2_physics": 32 + 32 + 32,
+               "apply": 32 + 16 + 33 + 32, "reduce": 32 + 1}
+
+
+def bytes_per_cell(kind, tile):
+    if kind not in STATE_BYTES:
+        return None
+    geometry = (49 if tile == "14x16" else 1) if kind.startswith("stage") else 0
+    return STATE_BYTES[kind] + geometry
+
+
 THROTTLE_BITS = {0x1: "gpu_idle", 0x2: "applications_clocks_setting", 0x4: "sw_power_cap", 0x8: "hw_slowdown",
                  0x10: "sync_boost", 0x20: "sw_thermal_slowdown", 0x40: "hw_thermal_slowdown",
                  0x80: "hw_power_brake_slowdown", 0x100: "display_clock_setting"}
@@ -338,7 +348,7 @@ def run_ours(args, rank, world, local_rank):
     launches_per_step = kn / (args.steps * SOLVER_STEPS)
     avg_ms = step_ms * (kms / total_ms) / launches_per_step
     peak, peak_kind = measured_peak()
-    bpc = BYTES_PER_CELL.get(kind)
+    bpc = bytes_per_cell(kind, tile_name)
     achieved = bpc * cells / (avg_ms * 1e-3) / 1e9 if bpc else None
     traffic_pc = profiled_traffic(kind)
 
@@ -499,7 +509,7 @@ def run_batched(args, local_rank, rank=0, world=1):
     for s in setups:
         sizes[f"{s.Nx}x{s.Nr}"] = sizes.get(f"{s.Nx}x{s.Nr}", 0) + 1
     peak, src = measured_peak()
-    bpc = BYTES_PER_CELL["stage1"] + BYTES_PER_CELL["stage2_physics"]
+    bpc = bytes_per_cell("stage1", tile) + bytes_per_cell("stage2_physics", tile)
     instances = int(replicas.sum_over_ranks(len(setups), dev))
     classes = None
     if world == 1 and not args.no_classes:
@@ -625,9 +635,10 @@ def t_setups_end(s, t_end_s):
 def run_large_grid(args):
     """HBM-resident sweep point: the plain cold-gas nozzle on a 4096 x 1536
     grid (6.3 M cells; one state copy is 201 MB, beyond the 126 MB L2), two
-    kernels per step. Achieved GB/s = algorithmic bytes per cell-step (258 B:
-    stage 1 reads 32 + 49, writes 32; stage 2 reads 32 + 32 + 49, writes 32)
-    x cell-steps/s, device time from CUDA events."""
+    kernels per step. Achieved GB/s = algorithmic bytes per cell-step (162 B:
+    stage 1 reads 32 + 1, writes 32; stage 2 reads 32 + 32 + 1, writes 32; 49
+    in place of the 1 with 14x16 tiles) x cell-steps/s, device time from CUDA
+    events."""
     import torch
     rn = ge.load_package()
     from rocket_nozzle_cfd_solver_b200.configs import plain_small
@@ -658,12 +669,12 @@ def run_large_grid(args):
     cells = s.Nx * s.Nr
     rate = cells * n * args.steps / (ms * 1e-3)
     peak, src = measured_peak()
-    bpc = BYTES_PER_CELL["stage1"] + BYTES_PER_CELL["stage2"]
+    bpc = bytes_per_cell("stage1", tile) + bytes_per_cell("stage2", tile)
     kern = {}
     for k in ("stage1", "stage2"):
         kms, kn = prof[k]
         if kn:
-            gbs = BYTES_PER_CELL[k] * cells / (kms / kn * 1e-3) / 1e9
+            gbs = bytes_per_cell(k, tile) * cells / (kms / kn * 1e-3) / 1e9
             kern[k] = {"avg_launch_us": 1e3 * kms / kn, "achieved_gbs": gbs, "frac": gbs / peak}
     g.close()
     return {"workload": "plain cold-gas nozzle 4096x1536 (inviscid, 2 kernels per step)", "cells": cells,
