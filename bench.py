@@ -426,7 +426,7 @@ def run_batched(args, local_rank, rank=0, world=1):
     """The batched workload: `--batch-instances` seeded nozzles (grids drawn
     from 128x48 .. 1024x384, expansion 4-40, p0 10-100 bar, gamma 1.2/1.4,
     altitude 0-30 km, all viscous) stepped by one SolverBatch (one launch per
-    kernel kind per step, 6-step periods replayed from a CUDA graph, tile shape
+    kernel kind per step, 6 steps at a time replayed from a CUDA graph, tile shape
     from the batch autotuner), against the same handles stepped one at a time
     with rn_step. Both are device times from CUDA events; the batch's state
     (~1 GB with geometry) is far larger than L2, so no flush is needed."""

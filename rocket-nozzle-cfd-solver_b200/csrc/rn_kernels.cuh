@@ -182,7 +182,7 @@ __host__ __device__ inline void batch_ring(const BatchInst& d, const BatchPhase&
 //   exact -- IEEE division and square root: every float operation rounds as
 //            written, so the state matches the CPU oracle bit for bit wherever
 //            pow/exp/log/sin/cos agree with the host's libm;
-//   fast  -- the hardware's approximate division (div.full) and square root
+//   fast  -- the hardware's approximate reciprocal and square root
 //            (within 2 ulp, the latitude GLSL highp gives the reference's
 //            shaders); agrees with the oracle to ~1e-6 relative L2.
 // A solver handle launches through one of the two sets; `tile` selects the

@@ -1,8 +1,8 @@
 // rn_tma.cuh -- tensor-memory-accelerator (TMA) staging of a tile's halo.
 //
 // The stage kernels start by copying the raw state of their tile plus its
-// 2-cell halo (the A and B float4 planes) and the matching block of the solid
-// mask from global memory into shared memory with 2-D tiled bulk tensor
+// 2-cell halo (the A and B float4 planes) and the matching block of the cell
+// classes from global memory into shared memory with 2-D tiled bulk tensor
 // copies (cp.async.bulk.tensor), issued by one thread and completed on an
 // mbarrier. Cells outside the grid arrive as zeros (the copy's out-of-bounds
 // fill); the ghost-cell pass (FS_PRIM, solver.js:56-126) then overwrites them
@@ -21,7 +21,7 @@ namespace rn {
 struct TileMaps {
   CUtensorMap a[3];     // state ring slots, plane A: box (PX x PY) float4 as 4*PX floats
   CUtensorMap b[3];     // plane B
-  CUtensorMap mask;     // row-pitched copy of the solid mask: box (MW x PY) bytes
+  CUtensorMap mask;     // row-pitched cell classes (CellClass): box (MW x PY) bytes
   CUtensorMap geoM;     // geoM with a 1-cell ring: box (TX+2) x (TY+2) float4 (shapes that stage it)
   CUtensorMap geoG;     // geoG of the tile: box TX x TY float4
 };
