@@ -507,13 +507,18 @@ RN_DEV void sub4(float4& L, float ae, float4 fe, float aw, float4 fw) {
 
 // L of a cell whose x-faces have area ax and whose south and north faces have
 // areas as_ and as_ + 1 (an uncut cell), after sub4's of both directions from
-// L = 0. The fast variant forms the differences first: two packed operations a
-// pair for x, three for r, where sub4 takes twelve scalar ones.
+// L = 0. The fast variant takes sub4's products and sums in lane pairs: ten
+// packed operations where sub4 takes 24 scalar ones. Each product a f is rounded
+// and its partner fused, as sub4's are: forming the differences fe - fw and
+// fn - fs first takes as many operations, but then G's update, the difference of
+// its flux and G times the velocity's, came out 1.38 times as far from a 64-bit
+// run (128x48 grids, 120 steps: 1.09e-6 against 7.9e-7).
 RN_DEV float4 box4(float ax, float as_, float4 fw, float4 fe, float4 fs, float4 fn) {
 #ifdef RN_FAST
-  const float2 x = make_float2(-ax, -ax), r = make_float2(as_, as_);
-  const float2 xl = mul2(x, sub2(lo2(fe), lo2(fw))), xh = mul2(x, sub2(hi2(fe), hi2(fw)));
-  const float2 rl = madd2(r, sub2(lo2(fn), lo2(fs)), lo2(fn)), rh = madd2(r, sub2(hi2(fn), hi2(fs)), hi2(fn));
+  const float2 xw = make_float2(ax, ax), xe = make_float2(-ax, -ax);
+  const float2 rs = make_float2(-as_, -as_), rn = make_float2(as_ + 1.0f, as_ + 1.0f);
+  const float2 xl = madd2(xe, lo2(fe), mul2(xw, lo2(fw))), xh = madd2(xe, hi2(fe), mul2(xw, hi2(fw)));
+  const float2 rl = madd2(rn, lo2(fn), mul2(rs, lo2(fs))), rh = madd2(rn, hi2(fn), mul2(rs, hi2(fs)));
   return cat4(sub2(xl, rl), sub2(xh, rh));
 #else
   float4 L = make_float4(0.f, 0.f, 0.f, 0.f);

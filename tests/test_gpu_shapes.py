@@ -136,3 +136,37 @@ def test_spray_steps_on_each_default_shape(rn, oracle, Nx, Nr):
     alive = lambda p: np.asarray(p).reshape(-1, 4)[:, 1] > 0  # noqa: E731
     assert np.array_equal(alive(g.spray.readParcels()["PB"]), alive(o.readParcels()["PB"]))
     g.close()
+
+
+@pytest.mark.parametrize("kind,Nx,Nr,precision", [("plain_small", 101, 38, "fast"), ("viscous_plume", 128, 48, "fast"),
+                                                  ("viscous_plume", 128, 48, "exact"), ("injector_spray", 192, 72, "exact")])
+def test_uncut_cells_round_as_the_general_path(rn, kind, Nx, Nr, precision):
+    """Uncut cells take their net fluxes from their four faces directly where
+    the general path sums a cut-cell group; both round every product and sum
+    alike, in fast precision too (but for the oxidiser's scalar sums, which the
+    compiler contracts as it likes: sprays in exact precision). A wall vector of
+    1e-7 in every uncut cell (below the 1e-6 at which a wall counts) sends the
+    same flow through the general path: the states are equal, values below the
+    smallest normal float apart (fast precision flushes those to zero or not,
+    as an operation comes packed or alone)."""
+    from rocket_nozzle_cfd_solver_b200 import configs
+    s = rn.build_sim_setup(dict(getattr(configs, kind)(Nx, Nr)[0], startMode="burst"))
+    init = s.initialState()
+    gG = np.array(s.geo["geoG"], np.float32).reshape(-1, 4)
+    gG[:, 2] = np.where((gG[:, 2] == 0) & (gG[:, 3] == 0), np.float32(1e-7), gG[:, 2])
+    outs = []
+    for geo in (s.geo, dict(s.geo, geoG=gG.reshape(-1))):
+        g = rn.GPUSolver(s.Nx, s.Nr)
+        g.setPrecision(precision)
+        g.setTile("16x15")
+        g.setGeometry(geo)
+        g.setState(init["A"], init["B"])
+        if s.injector is not None:
+            rn.GPUSpray(g).resize()
+            g.spray.setInjector(s.injector)
+        g.step(60, s.P)
+        outs.append(g.readAll())
+        g.close()
+    for k in ("A", "B"):
+        a, b = (np.where(np.abs(o[k]) < np.finfo(np.float32).tiny, 0, o[k]) for o in outs)
+        assert np.array_equal(a, b), (k, np.abs(a - b).max(), (a != b).sum())
