@@ -389,6 +389,19 @@ int rn_build_member_lists(rn_solver* h) {
   return RN_OK;
 }
 
+int rn_fit_member_lists(rn_solver* h) {
+  if (!h->autoShape) return rn_build_member_lists(h);
+  h->shape = rn_auto_shape(h->Nx, h->Nr, h->numSMs);
+  int rc = rn_build_member_lists(h);
+  const int named = rn_default_tile(h->Nx, h->Nr, h->numSMs);
+  // long lists cost 16x16 blocks their fourth place on an SM
+  if (h->shape != named && (rc != RN_OK || (h->shape == RN_TILE_16x16 && h->maxX > XSMALL))) {
+    h->shape = named;
+    rc = rn_build_member_lists(h);
+  }
+  return rc;
+}
+
 namespace {
 
 cudaEvent_t prof_event(rn_solver* h) {
@@ -571,13 +584,7 @@ int rn_set_geometry(rn_handle h, const uint8_t* mask, const float* geoA, const f
   for (size_t k = 0; k < N; k++) h->hostMask[k] = mask[k] ? 1 : 0;
   h->hostGeoM.assign(geoM, geoM + 4 * N);
   const int oldShape = h->shape;
-  if (h->autoShape) h->shape = rn_auto_shape(Nx, Nr, h->numSMs);
-  int rc = rn_build_member_lists(h);
-  if (h->autoShape && h->shape == RN_TILE_16x16 && (rc != RN_OK || h->maxX > XSMALL)) {
-    // long lists cost 16x16 blocks their fourth place on an SM
-    h->shape = RN_TILE_16x15;
-    rc = rn_build_member_lists(h);
-  }
+  int rc = rn_fit_member_lists(h);
   if (rc != RN_OK) {
     std::string msg = g_err;
     h->shape = oldShape;

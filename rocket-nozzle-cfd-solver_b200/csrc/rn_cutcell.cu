@@ -447,7 +447,7 @@ int rn_build_geometry(rn_handle h, const rn_cut_spec* sp, rn_cut_stats* stats) {
   h->hostMask = mask;
   h->hostGeoM.resize(size_t(N) * 4);
   std::memcpy(h->hostGeoM.data(), gm.data(), sizeof(float4) * N);
-  int rc = rn_build_member_lists(h);
+  int rc = rn_fit_member_lists(h);
   if (rc != RN_OK) return rc;
   rc = rn_classes_refresh(h);
   if (rc != RN_OK) return rc;

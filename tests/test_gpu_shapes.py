@@ -170,3 +170,102 @@ def test_uncut_cells_round_as_the_general_path(rn, kind, Nx, Nr, precision):
     for k in ("A", "B"):
         a, b = (np.where(np.abs(o[k]) < np.finfo(np.float32).tiny, 0, o[k]) for o in outs)
         assert np.array_equal(a, b), (k, np.abs(a - b).max(), (a != b).sum())
+
+
+def longest_list(geoM, Nx, Nr, TX, TY):
+    """Most cells outside one TX x TY tile that belong to a group with a cell inside it."""
+    gM = np.asarray(geoM).reshape(Nr, Nx, 4)
+    lists = {}
+    for j, i in zip(*np.nonzero(gM[..., 2])):
+        bits = int(gM[j, i, 2]) & 15
+        group = [(j, i)] + [(j + dj, i + di) for b, dj, di in ((1, 0, -1), (2, 0, 1), (4, -1, 0), (8, 1, 0)) if bits & b]
+        for a in group:
+            t = (a[0] // TY, a[1] // TX)
+            lists.setdefault(t, set()).update(c for c in group if (c[0] // TY, c[1] // TX) != t)
+    return max(map(len, lists.values()), default=0)
+
+
+def channel_setup(Nx, Nr):
+    """Fluid with solid blocks around a channel one cell and two slivers wide,
+    which runs along three sides of the 16 x 16 tile at (16, 16): each channel
+    cell and its outer sliver are members outside that tile of a group with a
+    sliver inside it."""
+    from types import SimpleNamespace
+    from rocket_nozzle_cfd_solver_b200 import cutcell
+    blocks = ((16.4, 40, 16.4, 31.6), (12, 14.6, 12, 36), (12, 40, 12, 14.6), (12, 40, 33.4, 36))
+    contour = SimpleNamespace(xe=-1.0, xt=0.0, Rt=0.0, radiusAt=lambda x: 0.0)
+    inp = {"Nx": Nx, "Nr": Nr, "dx": 1.0, "contour": contour, "tw": 0.0, "base": False, "xBase": 0.0, "bodyR": 0.0,
+           "solids": [dict(zip(("x0", "x1", "r0", "r1"), b)) for b in blocks]}
+    return {"cutInput": inp, "contour": contour, "rinCol": np.zeros(Nx, np.float32), "iExit": 0, "dx": 1.0,
+            "geo": cutcell.build_cut_geometry(inp)}
+
+
+def test_lists_too_long_for_the_small_shape(rn):
+    """An unset handle takes a geometry whose lists fit its named shape (14x16)
+    but not the 10x10 one its size would run: 72 members outside the 10x10
+    tile at (10, 10), where a tile may list 64."""
+    from rocket_nozzle_cfd_solver_b200 import configs
+    s = rn.build_sim_setup(configs.plain_small(96, 36)[0])
+    Nx, Nr = s.Nx, s.Nr
+    rows = np.arange(Nr + 1, dtype=np.float32)[:, None]
+    gA, gG, gM = np.zeros((Nr + 1, Nx + 1, 4), np.float32), np.zeros((Nr, Nx, 4), np.float32), np.zeros((Nr, Nx, 4), np.float32)
+    gA[..., 2], gA[..., 3] = rows + 0.5, rows
+    gA[Nr, :, 2] = gA[:, Nx, 3] = 0
+    gG[..., 0], gG[..., 1], gM[..., 3] = rows[:Nr] + 0.5, 1, 0.17
+    groups = [((9, j), (10, j), (8, j)) for j in range(10, 20)] + [((20, j), (19, j), (21, j)) for j in range(10, 20)]
+    groups += [((i, 9), (i, 10), (i, 8)) for i in range(11, 19)] + [((i, 20), (i, 19), (i, 21)) for i in range(11, 19)]
+    bit = {(-1, 0): 1, (1, 0): 2, (0, -1): 4, (0, 1): 8}
+    for (hi, hj), *slaves in groups:
+        for i, j in slaves:
+            gM[hj, hi, 2] += bit[i - hi, j - hj]
+            gM[j, i, :2] = hi - i, hj - j
+        cells = [(hi, hj)] + slaves
+        total = sum(gG[j, i].copy() for i, j in cells)
+        for i, j in cells:
+            gG[j, i] = total
+    assert longest_list(gM, Nx, Nr, 10, 10) > 64 >= longest_list(gM, Nx, Nr, 14, 16)
+    geo = dict(s.geo, mask=np.zeros(Nx * Nr, np.uint8), geoA=gA.reshape(-1), geoG=gG.reshape(-1), geoM=gM.reshape(-1))
+    init = s.initialState()
+    outs = []
+    for tile in (None, "14x16"):
+        g = rn.GPUSolver(Nx, Nr)
+        g.setPrecision("exact")
+        if tile:
+            g.setTile(tile)
+        g.setGeometry(geo)
+        g.setState(init["A"], init["B"])
+        g.step(9, s.P)
+        outs.append(g.readAll())
+        g.setGeometry(s.geo)                     # and back to one that fits the small shape
+        g.setState(init["A"], init["B"])
+        g.step(9, s.P)
+        outs.append(g.readAll())
+        g.close()
+    for a, b in zip(outs[:2], outs[2:]):
+        assert np.array_equal(a["A"], b["A"]) and np.array_equal(a["B"], b["B"])
+
+
+@pytest.mark.parametrize("build", [False, True])
+def test_lists_too_long_for_16x16(rn, build):
+    """An unset handle whose size runs 16x16 tiles takes a geometry whose lists
+    fit 16x15 only, uploaded or built on the device."""
+    from rocket_nozzle_cfd_solver_b200 import configs
+    s = rn.build_sim_setup(configs.plain_small(1024, 287)[0])
+    c = channel_setup(s.Nx, s.Nr)
+    assert longest_list(c["geo"]["geoM"], s.Nx, s.Nr, 16, 16) > 64 >= longest_list(c["geo"]["geoM"], s.Nx, s.Nr, 16, 15)
+    init = s.initialState()
+    outs = []
+    for tile in (None, "16x15"):
+        g = rn.GPUSolver(s.Nx, s.Nr)
+        g.setPrecision("exact")
+        if tile:
+            g.setTile(tile)
+        if build:
+            g.buildGeometry(c)
+        else:
+            g.setGeometry(c["geo"])
+        g.setState(init["A"], init["B"])
+        g.step(5, s.P)
+        outs.append(g.readAll())
+        g.close()
+    assert np.array_equal(outs[0]["A"], outs[1]["A"]) and np.array_equal(outs[0]["B"], outs[1]["B"])
