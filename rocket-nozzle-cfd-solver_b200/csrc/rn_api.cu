@@ -389,7 +389,10 @@ int rn_build_member_lists(rn_solver* h) {
   return RN_OK;
 }
 
-int rn_fit_member_lists(rn_solver* h) {
+// Member lists of a new topology: while nobody set h's tile shape, for the
+// shape that suits its grid, or the one it is named by where that one's lists
+// are too long.
+static int fit_member_lists(rn_solver* h) {
   if (!h->autoShape) return rn_build_member_lists(h);
   h->shape = rn_auto_shape(h->Nx, h->Nr, h->numSMs);
   int rc = rn_build_member_lists(h);
@@ -400,6 +403,20 @@ int rn_fit_member_lists(rn_solver* h) {
     rc = rn_build_member_lists(h);
   }
   return rc;
+}
+
+int rn_set_topology(rn_solver* h, std::vector<uint8_t> mask, std::vector<float> geoM) {
+  const int shape = h->shape;
+  h->hostMask.swap(mask);
+  h->hostGeoM.swap(geoM);
+  const int rc = fit_member_lists(h);
+  if (rc == RN_OK) return RN_OK;
+  const std::string msg = g_err;
+  h->shape = shape;
+  h->hostMask.swap(mask);
+  h->hostGeoM.swap(geoM);
+  rn_build_member_lists(h);
+  return fail(rc, msg);
 }
 
 namespace {
@@ -578,21 +595,10 @@ int rn_set_geometry(rn_handle h, const uint8_t* mask, const float* geoA, const f
       return fail(RN_ERR_ARG, "rn_set_geometry: slave bit of cell " + std::to_string(k) + " points outside the grid");
   }
   const size_t N = size_t(Nx) * Nr, NF = size_t(Nx + 1) * (Nr + 1);
-  std::vector<uint8_t> oldMask = std::move(h->hostMask);
-  std::vector<float> oldGeoM = std::move(h->hostGeoM);
-  h->hostMask.resize(N);
-  for (size_t k = 0; k < N; k++) h->hostMask[k] = mask[k] ? 1 : 0;
-  h->hostGeoM.assign(geoM, geoM + 4 * N);
-  const int oldShape = h->shape;
-  int rc = rn_fit_member_lists(h);
-  if (rc != RN_OK) {
-    std::string msg = g_err;
-    h->shape = oldShape;
-    h->hostMask = std::move(oldMask);
-    h->hostGeoM = std::move(oldGeoM);
-    rn_build_member_lists(h);
-    return fail(rc, msg);
-  }
+  std::vector<uint8_t> hostMask(N);
+  for (size_t k = 0; k < N; k++) hostMask[k] = mask[k] ? 1 : 0;
+  int rc = rn_set_topology(h, std::move(hostMask), std::vector<float>(geoM, geoM + 4 * N));
+  if (rc != RN_OK) return rc;
   rc = rn_set_mask(h, mask);
   if (rc != RN_OK) return rc;
   CK(cudaMemcpyAsync(h->geoA, geoA, sizeof(float4) * NF, cudaMemcpyHostToDevice, h->stream));

@@ -238,7 +238,7 @@ __global__ void k_sliver_flags(CutDev c, uint8_t* flags) {
 
 struct OutDev {
   float4* geoA;
-  float4* geoG;
+  float4* geoG;       // may be null: the topology alone
   float4* geoM;
   uint8_t* mask;
   float4* jw;
@@ -334,7 +334,7 @@ __global__ void k_groups(CutDev c, OutDev o) {
     if (x > o.xt + 0.5 * o.Rt && Rin - r < fmax(2 * o.dx, delta)) M.z = float(double(M.z) + 16.0);
   }
   M.w = float(l);
-  o.geoG[k] = G;
+  if (o.geoG) o.geoG[k] = G;
   o.geoM[k] = M;
   o.mask[k] = sol ? 1 : 0;
 }
@@ -374,6 +374,7 @@ int rn_build_geometry(rn_handle h, const rn_cut_spec* sp, rn_cut_stats* stats) {
   const size_t oCol = take(sizeof(float) * 2 * Nx), oU8 = take(size_t(N) * 4), oHost = take(sizeof(int) * N);
   const size_t oF = take(sizeof(float) * 3 * size_t(N)), oFace = take(sizeof(float) * 2 * size_t(NF));
   const size_t oSl = take(sizeof(int) * (size_t(N) + 1)), oCnt = take(sizeof(unsigned) * 4);
+  const size_t oTopM = take(sizeof(float4) * N), oTopMask = take(size_t(N));
   size_t cubBytes = 0;
   cub::DeviceSelect::Flagged(nullptr, cubBytes, thrust::counting_iterator<int>(0), (const uint8_t*)nullptr,
                              (int*)nullptr, (int*)nullptr, N, s);
@@ -405,6 +406,11 @@ int rn_build_geometry(rn_handle h, const rn_cut_spec* sp, rn_cut_stats* stats) {
   o.counts = reinterpret_cast<unsigned*>(base + oCnt);
   o.rinCol = reinterpret_cast<float*>(base + oRinCol);
   o.dx = sp->dx; o.xt = sp->xt; o.xe = sp->xe; o.Rt = sp->Rt; o.iExit = sp->iExit;
+  OutDev top = o;
+  top.geoG = nullptr;
+  top.geoM = reinterpret_cast<float4*>(base + oTopM);
+  top.mask = reinterpret_cast<uint8_t*>(base + oTopMask);
+  top.counts = o.counts + 2;
   cudaError_t e = cudaSuccess;
   auto ck = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
   ck(cudaMemcpyAsync((void*)c.Rtab, sp->Rtab, sizeof(float) * nTab, cudaMemcpyHostToDevice, s));
@@ -426,38 +432,41 @@ int rn_build_geometry(rn_handle h, const rn_cut_spec* sp, rn_cut_stats* stats) {
     ck(cub::DeviceSelect::Flagged(base + oCub, cb, thrust::counting_iterator<int>(0), flags, sliv, nSliv, N, s));
     k_merge<<<1, 32, 0, s>>>(c, sliv, nSliv);
     k_solid_faces<<<gL, b2, 0, s>>>(c);
-    k_geoA<<<gL, b2, 0, s>>>(c, o);
-    k_groups<<<gC, b2, 0, s>>>(c, o);
-    k_jwall<<<(Nx + 127) / 128, 128, 0, s>>>(c, o);
+    // the topology into scratch first: the handle's planes are written once its
+    // member lists are known to fit
+    k_groups<<<gC, b2, 0, s>>>(c, top);
     ck(cudaGetLastError());
-    h->launches += 11;
   }
   // host copies of the topology for the per-tile member lists
   unsigned cnt[4] = {0, 0, 0, 0};
   std::vector<uint8_t> mask(N);
-  std::vector<float4> gm(N);
+  std::vector<float> gm(size_t(N) * 4);
   if (e == cudaSuccess) {
-    ck(cudaMemcpyAsync(mask.data(), h->mask, N, cudaMemcpyDeviceToHost, s));
-    ck(cudaMemcpyAsync(gm.data(), h->geoM, sizeof(float4) * N, cudaMemcpyDeviceToHost, s));
+    ck(cudaMemcpyAsync(mask.data(), top.mask, N, cudaMemcpyDeviceToHost, s));
+    ck(cudaMemcpyAsync(gm.data(), top.geoM, sizeof(float4) * N, cudaMemcpyDeviceToHost, s));
     ck(cudaMemcpyAsync(cnt, o.counts, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+    ck(cudaStreamSynchronize(s));
+  }
+  int rc = RN_OK;
+  if (e == cudaSuccess) rc = rn_set_topology(h, std::move(mask), std::move(gm));
+  if (e == cudaSuccess && rc == RN_OK) {
+    k_geoA<<<gL, b2, 0, s>>>(c, o);
+    k_groups<<<gC, b2, 0, s>>>(c, o);
+    k_jwall<<<(Nx + 127) / 128, 128, 0, s>>>(c, o);
+    ck(cudaGetLastError());
+    h->launches += 12;
+    rc = rn_classes_refresh(h);
+    // a step kernel's copies of the classes may start before the kernel ahead of
+    // it in the stream has completed
     ck(cudaStreamSynchronize(s));
   }
   cudaFree(base);
   if (e != cudaSuccess) return rn_record_cuda(e, "rn_build_geometry");
-  h->hostMask = mask;
-  h->hostGeoM.resize(size_t(N) * 4);
-  std::memcpy(h->hostGeoM.data(), gm.data(), sizeof(float4) * N);
-  int rc = rn_fit_member_lists(h);
   if (rc != RN_OK) return rc;
-  rc = rn_classes_refresh(h);
-  if (rc != RN_OK) return rc;
-  // a step kernel's copies of the classes may start before the kernel ahead of
-  // it in the stream has completed
-  RN_CK(cudaStreamSynchronize(h->stream));
   h->wvalid = false;
   if (stats) {
-    stats->nCut = int(cnt[0]);
-    stats->nMerged = int(cnt[1]);
+    stats->nCut = int(cnt[2]);
+    stats->nMerged = int(cnt[3]);
   }
   return RN_OK;
 }

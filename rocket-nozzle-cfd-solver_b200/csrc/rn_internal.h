@@ -147,10 +147,9 @@ int rn_auto_shape(int Nx, int Nr, int numSMs);
 int rn_use_shape(rn_solver* h, int shape);
 // (Re)build the per-tile member lists of `h` for its current tile shape.
 int rn_build_member_lists(rn_solver* h);
-// The same for a new topology: while nobody set h's tile shape, first takes the
-// shape that suits its grid, or the one it is named by where that one's lists
-// are too long.
-int rn_fit_member_lists(rn_solver* h);
+// Takes a new topology (solid mask, geoM) as h's host copy, chooses the shape
+// for it and builds its member lists; on failure h keeps the one it had.
+int rn_set_topology(rn_solver* h, std::vector<uint8_t> mask, std::vector<float> geoM);
 // Make h->wmax[h->wslot] the wave-speed max of the current state if it is not.
 int rn_ensure_wave_speed(rn_solver* h);
 // Takes h out of its batch, if any (rn_batch.cu).

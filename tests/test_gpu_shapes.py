@@ -185,14 +185,18 @@ def longest_list(geoM, Nx, Nr, TX, TY):
     return max(map(len, lists.values()), default=0)
 
 
-def channel_setup(Nx, Nr):
-    """Fluid with solid blocks around a channel one cell and two slivers wide,
-    which runs along three sides of the 16 x 16 tile at (16, 16): each channel
-    cell and its outer sliver are members outside that tile of a group with a
-    sliver inside it."""
+CHANNEL = ((16.4, 40, 16.4, 31.6), (12, 14.6, 12, 36), (12, 40, 12, 14.6), (12, 40, 33.4, 36))
+POCKET = ((20, 76, 5, 14.7), (20, 76, 30.3, 40), (20, 31.7, 18, 26))
+
+
+def blocks_setup(Nx, Nr, blocks):
+    """Fluid around solid blocks (x0, x1, r0, r1), in cells. CHANNEL leaves a
+    channel one cell and two slivers wide along three sides of the 16 x 16 tile
+    at (16, 16): each channel cell and its outer sliver are members outside that
+    tile of a group with a sliver inside it. POCKET has slivers just outside the
+    32 x 15 tile at (32, 15) merged into it: 32 below, 32 above, 8 on the left."""
     from types import SimpleNamespace
     from rocket_nozzle_cfd_solver_b200 import cutcell
-    blocks = ((16.4, 40, 16.4, 31.6), (12, 14.6, 12, 36), (12, 40, 12, 14.6), (12, 40, 33.4, 36))
     contour = SimpleNamespace(xe=-1.0, xt=0.0, Rt=0.0, radiusAt=lambda x: 0.0)
     inp = {"Nx": Nx, "Nr": Nr, "dx": 1.0, "contour": contour, "tw": 0.0, "base": False, "xBase": 0.0, "bodyR": 0.0,
            "solids": [dict(zip(("x0", "x1", "r0", "r1"), b)) for b in blocks]}
@@ -251,7 +255,7 @@ def test_lists_too_long_for_16x16(rn, build):
     fit 16x15 only, uploaded or built on the device."""
     from rocket_nozzle_cfd_solver_b200 import configs
     s = rn.build_sim_setup(configs.plain_small(1024, 287)[0])
-    c = channel_setup(s.Nx, s.Nr)
+    c = blocks_setup(s.Nx, s.Nr, CHANNEL)
     assert longest_list(c["geo"]["geoM"], s.Nx, s.Nr, 16, 16) > 64 >= longest_list(c["geo"]["geoM"], s.Nx, s.Nr, 16, 15)
     init = s.initialState()
     outs = []
@@ -265,6 +269,35 @@ def test_lists_too_long_for_16x16(rn, build):
         else:
             g.setGeometry(c["geo"])
         g.setState(init["A"], init["B"])
+        g.step(5, s.P)
+        outs.append(g.readAll())
+        g.close()
+    assert np.array_equal(outs[0]["A"], outs[1]["A"]) and np.array_equal(outs[0]["B"], outs[1]["B"])
+
+
+def test_refused_built_geometry_leaves_the_handle_as_it_was(rn):
+    """rn_build_geometry of a geometry that the set tile shape cannot hold fails
+    and changes nothing: the planes read back as before, and the handle steps
+    as one that was never asked (its classes, lists and planes go together)."""
+    from rocket_nozzle_cfd_solver_b200 import configs
+    s = rn.build_sim_setup(configs.viscous_plume(96, 45)[0])
+    c = blocks_setup(s.Nx, s.Nr, POCKET)
+    assert longest_list(c["geo"]["geoM"], s.Nx, s.Nr, 32, 15) > 64
+    init = s.initialState()
+    outs = []
+    for ask in (False, True):
+        g = rn.GPUSolver(s.Nx, s.Nr)
+        g.setPrecision("exact")
+        g.setTile("32x15")
+        g.setGeometry(s.geo)
+        g.setState(init["A"], init["B"])
+        g.step(3, s.P)
+        if ask:
+            before = g.readGeometry()
+            with pytest.raises(rn.solver.RnError):
+                g.buildGeometry(c)
+            after = g.readGeometry()
+            assert all(np.array_equal(before[k], after[k]) for k in before)
         g.step(5, s.P)
         outs.append(g.readAll())
         g.close()
