@@ -249,7 +249,10 @@ int rn_batch_step(rn_batch b, int n);
 int rn_batch_run(rn_batch b, const double* t_end, int chunk, long long max_steps, long long* steps);
 int rn_batch_sync(rn_batch b);
 /* tile shape of the batch's launches (RN_TILE_*); RN_TILE_16x15 until set, run
- * as 16 x 16 where the members' grids need clearly fewer tiles of that */
+ * as 16 x 16 where that suits the members' grids and geometry better (a member's
+ * results are the same either way; in fast precision values below the smallest
+ * normal float may be flushed to zero in one and kept in the other). A member
+ * that leaves has the shape it is named by from its next step on. */
 int rn_batch_set_tile(rn_batch b, int shape);
 /* times `steps` batch steps with each tile shape on copies of the members'
  * current states (states, step info and spray rings are restored), keeps the

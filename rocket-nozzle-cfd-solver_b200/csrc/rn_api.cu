@@ -182,6 +182,7 @@ int alloc_buffers(rn_solver* h, int Nx, int Nr) {
   h->cur = 0; h->stepIdx = 0; h->wslot = 0; h->wvalid = false; h->stepCount = 0;
   h->seed = 1;
   if (h->autoShape) h->shape = rn_auto_shape(Nx, Nr, h->numSMs);
+  else if (!h->batch) h->shape = h->tile;
   // empty topology (no groups) until a geometry is set
   h->hostMask.assign(N, 0);
   h->hostGeoM.assign(N * 4, 0.0f);
@@ -393,7 +394,11 @@ int rn_build_member_lists(rn_solver* h) {
 // shape that suits its grid, or the one it is named by where that one's lists
 // are too long.
 static int fit_member_lists(rn_solver* h) {
-  if (!h->autoShape) return rn_build_member_lists(h);
+  if (h->batch) return rn_batch_fit_member_lists(h);
+  if (!h->autoShape) {
+    h->shape = h->tile;
+    return rn_build_member_lists(h);
+  }
   h->shape = rn_auto_shape(h->Nx, h->Nr, h->numSMs);
   int rc = rn_build_member_lists(h);
   const int named = rn_default_tile(h->Nx, h->Nr, h->numSMs);
@@ -975,6 +980,11 @@ int rn_step(rn_handle h, int n, const rn_params* P) {
   const int perStep = 2 + (inj ? 2 : 0);
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cs = cudaStreamCaptureStatusNone;
+  // a handle that left a batch of another shape returns to the one it is named by
+  // (not in a caller's capture, which cannot hold the new lists' allocation)
+  if (!h->autoShape && h->shape != h->tile && cs == cudaStreamCaptureStatusNone &&
+      rn_use_shape(h, h->tile) != RN_OK)
+    h->tile = h->shape;                         // the lists fit the shape it has only
   if (h->prof == 2 && !inj && cs == cudaStreamCaptureStatusNone && n >= 2 * PROF_STEPS) {
     int rc = prof_graph_steps(h, P, n, done);
     if (rc != RN_OK) return rc;

@@ -51,6 +51,7 @@ struct rn_batch_t {
   int tile = RN_TILE_16x15;             // public name
   int shape = RN_TILE_16x15;            // what the kernels run; not `tile` only while autoShape
   bool autoShape = true;                // nobody set the tile shape
+  bool longLists = false;               // a member's lists are too long for 16x16
   Flags flags;
   std::vector<rn_solver*> members;
   std::vector<rn_params> params;
@@ -506,7 +507,8 @@ int use_shape(rn_batch_t* b, int shape) {
 }
 
 // Brings h, about to join, and the batch to one shape: the one set, or, while
-// nobody set one, the one that suits the members' grids and h's.
+// nobody set one, the one that suits the members' grids and h's. Lists above
+// XSMALL cost 16x16 blocks their fourth place on an SM.
 int join_shape(rn_batch_t* b, rn_solver* h) {
   if (b->autoShape) {
     long long t16 = tile_count(RN_TILE_16x16, h->Nx, h->Nr), t15 = tile_count(RN_TILE_16x15, h->Nx, h->Nr);
@@ -514,9 +516,13 @@ int join_shape(rn_batch_t* b, rn_solver* h) {
       t16 += tile_count(RN_TILE_16x16, q->Nx, q->Nr);
       t15 += tile_count(RN_TILE_16x15, q->Nx, q->Nr);
     }
-    if (prefer_16x16(t16, t15) && use_shape(b, RN_TILE_16x16) == RN_OK && rn_use_shape(h, RN_TILE_16x16) == RN_OK)
-      return RN_OK;
-    const int rc = use_shape(b, RN_TILE_16x15);   // (or 16x16's lists are too long)
+    if (!b->longLists && prefer_16x16(t16, t15)) {
+      b->longLists = use_shape(b, RN_TILE_16x16) != RN_OK || rn_use_shape(h, RN_TILE_16x16) != RN_OK ||
+                     h->maxX > XSMALL;
+      for (const rn_solver* q : b->members) b->longLists |= q->maxX > XSMALL;
+      if (!b->longLists) return RN_OK;
+    }
+    const int rc = use_shape(b, RN_TILE_16x15);
     if (rc != RN_OK) return rc;
   }
   return rn_use_shape(h, b->shape);
@@ -552,6 +558,15 @@ int release_members(rn_batch_t* b) {
 }
 
 }  // namespace
+
+int rn_batch_fit_member_lists(rn_solver* h) {
+  rn_batch_t* b = h->batch;
+  const int rc = rn_build_member_lists(h);
+  if (!b->autoShape || b->shape != RN_TILE_16x16 || (rc == RN_OK && h->maxX <= XSMALL)) return rc;
+  b->longLists = true;
+  const int rc15 = use_shape(b, RN_TILE_16x15);
+  return rc == RN_OK ? RN_OK : rc15;   // (where 16x15 cannot hold them either, 16x16 stays)
+}
 
 // Removes h from its batch (rn_destroy of a member).
 void rn_batch_detach(rn_solver* h) {
@@ -797,6 +812,7 @@ int rn_batch_remove(rn_batch b, rn_handle h) {
   b->members.erase(b->members.begin() + m);
   b->params.erase(b->params.begin() + m);
   b->fence.erase(b->fence.begin() + m);
+  b->longLists = false;
   h->batch = nullptr;
   return RN_OK;
 }

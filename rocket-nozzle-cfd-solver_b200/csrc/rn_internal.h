@@ -90,7 +90,8 @@ struct rn_solver {
   // tile shape of the stage/physics kernels and, per tile, the out-of-tile
   // members of its cut-cell groups (built from host copies of the topology)
   // (tile: the public name; shape: what its kernels run, TILE_TX/TILE_TY's index.
-  // They differ only while autoShape, i.e. until a caller sets the tile shape)
+  // They differ only while autoShape, i.e. until a caller sets the tile shape, in
+  // a batch whose shape nobody set, and from leaving one to the next step)
   int tile = RN_TILE_16x15, shape = RN_TILE_16x15;
   bool autoShape = true;
   rn::MemberHead* xhead = nullptr;
@@ -152,6 +153,10 @@ int rn_build_member_lists(rn_solver* h);
 int rn_set_topology(rn_solver* h, std::vector<uint8_t> mask, std::vector<float> geoM);
 // Make h->wmax[h->wslot] the wave-speed max of the current state if it is not.
 int rn_ensure_wave_speed(rn_solver* h);
+// Member lists of batch member h's new topology for the batch's shape; a batch
+// whose shape nobody set goes back to 16x15 where they are too long for 16x16
+// (rn_batch.cu).
+int rn_batch_fit_member_lists(rn_solver* h);
 // Takes h out of its batch, if any (rn_batch.cu).
 void rn_batch_detach(rn_solver* h);
 // Residual of the current state against the mark, into h->dRes[0..5], and the

@@ -302,3 +302,103 @@ def test_refused_built_geometry_leaves_the_handle_as_it_was(rn):
         outs.append(g.readAll())
         g.close()
     assert np.array_equal(outs[0]["A"], outs[1]["A"]) and np.array_equal(outs[0]["B"], outs[1]["B"])
+
+
+def test_batch_shape_follows_its_members_geometry(rn):
+    """A batch whose shape nobody set runs 16x16 tiles for these grids (2 waves
+    of blocks against 3). A member's new geometry whose lists fit 16x15 only is
+    taken all the same, uploaded or built, as is one set after leaving the batch
+    under the name 16x15; every member steps as a handle of its own."""
+    from rocket_nozzle_cfd_solver_b200 import configs
+    ss = [rn.build_sim_setup(configs.plain_small(*sz)[0]) for sz in ((1024, 287), (128, 48))]
+    big, small = ss
+    c = blocks_setup(big.Nx, big.Nr, CHANNEL)
+
+    def make(s, tile=None):
+        g = rn.GPUSolver(s.Nx, s.Nr)
+        g.setPrecision("exact")
+        if tile:
+            g.setTile(tile)
+        init = s.initialState()
+        g.setGeometry(s.geo)
+        g.setState(init["A"], init["B"])
+        return g
+
+    def same(a, b):
+        x, y = a.readAll(), b.readAll()
+        return np.array_equal(x["A"], y["A"]) and np.array_equal(x["B"], y["B"])
+    for build in (True, False):
+        batch = rn.SolverBatch()
+        members, alone = [make(s) for s in ss], [make(s, "16x15") for s in ss]
+        take = (lambda g: g.buildGeometry(c)) if build else (lambda g: g.setGeometry(c["geo"]))
+        for g, s in zip(members, ss):
+            batch.add(g, s.P)
+        batch.step(7)
+        for g, s in zip(alone, ss):
+            g.step(7, s.P)
+        take(members[0])                         # in the batch
+        take(alone[0])
+        batch.step(7)
+        for g, s in zip(alone, ss):
+            g.step(7, s.P)
+        assert all(same(g, h) for g, h in zip(members, alone))
+        batch.close()
+        for g in members + alone:
+            g.close()
+    batch = rn.SolverBatch()
+    g, h = make(big), make(big, "16x15")
+    batch.add(g, big.P)
+    batch.step(3)
+    batch.remove(g)
+    h.step(3, big.P)
+    assert g.tile == "16x15"
+    g.step(2, big.P)
+    h.step(2, big.P)
+    g.buildGeometry(c)                           # after leaving
+    h.buildGeometry(c)
+    g.step(3, big.P)
+    h.step(3, big.P)
+    assert same(g, h)
+    batch.close()
+    g.close()
+    h.close()
+
+
+@pytest.mark.parametrize("kind", ["plain_small", "viscous_plume", "injector_spray"])
+def test_a_members_bits_do_not_depend_on_its_companions(rn, kind):
+    """A batch whose shape nobody set moves from 16x16 tiles (the first member
+    alone) to 16x15 (with the second, which leaves no wave to save) between its
+    steps. In fast precision too each member ends with the bits of a handle set
+    to 16x15, values below the smallest normal float apart (flushed to zero or
+    not, as an operation comes packed or alone)."""
+    from rocket_nozzle_cfd_solver_b200 import configs
+    ss = [rn.build_sim_setup(dict(getattr(configs, kind)(*sz)[0], startMode="burst"))
+          for sz in ((1024, 287), (1024, 384))]
+
+    def make(s, tile=None):
+        g = rn.GPUSolver(s.Nx, s.Nr)
+        if tile:
+            g.setTile(tile)
+        init = s.initialState()
+        g.setGeometry(s.geo)
+        g.setState(init["A"], init["B"])
+        if s.injector is not None:
+            rn.GPUSpray(g).resize()
+            g.spray.setInjector(s.injector)
+        return g
+
+    batch = rn.SolverBatch()
+    members, alone = [make(s) for s in ss], [make(s, "16x15") for s in ss]
+    for k, s in enumerate(ss):
+        batch.add(members[k], s.P)
+        batch.step(15)
+        for h, t in list(zip(alone, ss))[:k + 1]:
+            h.step(15, t.P)
+    for g, h in zip(members, alone):
+        x, y = g.readAll(), h.readAll()
+        for p in ("A", "B"):
+            a, b = (np.where(np.abs(v[p]) < np.finfo(np.float32).tiny, 0, v[p]) for v in (x, y))
+            assert np.array_equal(a, b), (p, np.abs(a - b).max(), (a != b).sum())
+    batch.close()
+    for g in members + alone:
+        g.close()
