@@ -54,6 +54,8 @@ void rn_drop_step_graphs(rn_solver* h) {
   }
 }
 
+static int rn_default_tile(int Nx, int Nr, int numSMs);
+
 namespace {
 
 void free_buffers(rn_solver* h) {
@@ -181,8 +183,12 @@ int alloc_buffers(rn_solver* h, int Nx, int Nr) {
   CK(cudaMalloc(&h->sortTemp, h->sortTempBytes > 0 ? h->sortTempBytes : 16));
   h->cur = 0; h->stepIdx = 0; h->wslot = 0; h->wvalid = false; h->stepCount = 0;
   h->seed = 1;
-  if (h->autoShape) h->shape = rn_auto_shape(Nx, Nr, h->numSMs);
-  else if (!h->batch) h->shape = h->tile;
+  if (h->autoShape) {
+    h->tile = rn_default_tile(Nx, Nr, h->numSMs);
+    h->shape = rn_auto_shape(Nx, Nr, h->numSMs);
+  } else if (!h->batch) {
+    h->shape = h->tile;
+  }
   // empty topology (no groups) until a geometry is set
   h->hostMask.assign(N, 0);
   h->hostGeoM.assign(N * 4, 0.0f);
@@ -283,6 +289,8 @@ int rn_classes_refresh(rn_solver* h) {
   return RN_OK;
 }
 
+// The name of an unset shape: 14x16 (compiled for 3 blocks per SM) when the
+// grid's tiles are all resident at 3 per SM at once, else 16x15.
 static int rn_default_tile(int Nx, int Nr, int numSMs) {
   return tile_count(RN_TILE_14x16, Nx, Nr) <= 3 * numSMs ? RN_TILE_14x16 : RN_TILE_16x15;
 }
@@ -512,9 +520,6 @@ int rn_create(int Nx, int Nr, rn_handle* out) {
       kernels_ready = true;
     }
   }
-  // default tile shape: 14x16 (compiled for 3 blocks per SM) when the grid's
-  // tiles are all resident at 3 per SM at once, else 16x15
-  if (Nx > 0 && Nr > 0) h->tile = rn_default_tile(Nx, Nr, h->numSMs);
   int rc = alloc_buffers(h, Nx, Nr);
   if (rc != RN_OK) {
     std::string msg = g_err;

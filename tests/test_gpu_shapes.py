@@ -402,3 +402,17 @@ def test_a_members_bits_do_not_depend_on_its_companions(rn, kind):
     batch.close()
     for g in members + alone:
         g.close()
+
+
+def test_unset_name_follows_a_resize(rn):
+    """An unset handle is named by its present grid's size, a set one as set."""
+    g = rn.GPUSolver(128, 48)
+    for Nx, Nr in ((1024, 384), (128, 48), (2048, 512)):
+        h = rn.GPUSolver(Nx, Nr)
+        g.resize(Nx, Nr)
+        assert g.tile == h.tile, (Nx, Nr)
+        h.close()
+    g.setTile("16x8")
+    g.resize(128, 48)
+    assert g.tile == "16x8"
+    g.close()
