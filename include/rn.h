@@ -197,15 +197,18 @@ int rn_set_precision(rn_handle h, int mode);
 int rn_get_precision(rn_handle h, int* mode);
 
 /* Tile shape of the stage/physics kernels (a thread per cell):
- * RN_TILE_16x15, RN_TILE_16x16, RN_TILE_16x8, RN_TILE_32x15 or RN_TILE_14x16. A new handle
- * starts with RN_TILE_14x16 when the grid's 14 x 16 tiles number at most 3 per
- * SM (all resident at once), else with RN_TILE_16x15; until a shape is set its
- * kernels may run another that suits the grid's size better (10 x 10 on small
- * grids, 16 x 16 where it divides the height better) under that name.
- * rn_autotune times `steps` steps with each shape, that one included, on a copy
+ * RN_TILE_16x15, RN_TILE_16x16, RN_TILE_16x8, RN_TILE_32x15 or RN_TILE_14x16. A new
+ * (or, while none is set, resized) handle is named RN_TILE_14x16 when the grid's
+ * 14 x 16 tiles number at most 3 per SM (all resident at once), else
+ * RN_TILE_16x15; until a shape is set its kernels may run another that suits the
+ * grid's size better (10 x 10 on small grids, 16 x 16 where that saves a wave of
+ * blocks) under that name. Setting a shape, that name too, makes them run the
+ * shape named. rn_autotune times `steps` steps with each named shape on a copy
  * of the handle's current state (the state, step info and spray ring are
- * restored afterwards), keeps the fastest and returns its name in *chosen. No reference counterpart (the reference draws full-screen
- * fragment passes). */
+ * restored afterwards), sets the fastest and returns it in *chosen; the shape of
+ * an unset handle is not among them, and on small grids is faster than they
+ * are. No reference counterpart (the reference draws full-screen fragment
+ * passes). */
 #define RN_TILE_16x16 0
 #define RN_TILE_16x8 1
 #define RN_TILE_16x15 2   /* 16 x 15 cells on 256 threads */

@@ -1376,16 +1376,13 @@ int rn_autotune(rn_handle h, const rn_params* P, int steps, int* chosen) {
   const int prof = h->prof;
   h->prof = 0;
   cudaError_t e = copy_all(true);
-  // the public shapes, then the one an unset handle of this grid runs
-  const int unset = rn_auto_shape(h->Nx, h->Nr, h->numSMs);
-  int best = h->shape, rc = RN_OK;
+  const int oldShape = h->shape;
+  int best = -1, rc = RN_OK;
   float bestMs = 1e30f;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (e == cudaSuccess) e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
-  for (int q = 0; q <= NTILES && e == cudaSuccess && rc == RN_OK; q++) {
-    const int shape = q < NTILES ? q : unset;
-    if (q == NTILES && unset < NTILES) break;
+  for (int shape = 0; shape < NTILES && e == cudaSuccess && rc == RN_OK; shape++) {
     h->shape = shape;
     rc = rn_build_member_lists(h);
     if (rc != RN_OK) { rc = RN_OK; continue; }          // this shape cannot hold the geometry's lists
@@ -1411,9 +1408,12 @@ int rn_autotune(rn_handle h, const rn_params* P, int steps, int* chosen) {
   cudaFree(save);
   h->launches = launches;
   h->prof = prof;
-  h->shape = best;
-  h->autoShape = best >= NTILES;
-  h->tile = best < NTILES ? best : rn_default_tile(h->Nx, h->Nr, h->numSMs);
+  if (best < 0 || e != cudaSuccess || rc != RN_OK) {
+    h->shape = oldShape;                        // no shape was timed, or a trial failed: as before
+  } else {
+    h->shape = h->tile = best;
+    h->autoShape = false;
+  }
   int rc2 = rn_build_member_lists(h);
   if (e != cudaSuccess) return cuda_fail(e, "rn_autotune");
   if (rc != RN_OK) return rc;

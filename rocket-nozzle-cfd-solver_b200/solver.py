@@ -584,8 +584,8 @@ class GPUSolver:
         return {b: a for a, b in PRECISION.items()}[v.value]
 
     def setTile(self, shape):
-        """Tile shape of the stage/physics kernels: '16x15', '16x16', '16x8', '32x15' or '14x16' (a new handle
-        starts with '14x16' when its tiles number at most 3 per SM, else '16x15', and its kernels may run
+        """Tile shape of the stage/physics kernels: '16x15', '16x16', '16x8', '32x15' or '14x16' (an unset
+        handle is named '14x16' when its tiles number at most 3 per SM, else '16x15', and its kernels may run
         another shape under that name until one is set)."""
         _check(lib().rn_set_tile(self.h, TILES[shape]))
 
@@ -596,8 +596,9 @@ class GPUSolver:
         return {b: a for a, b in TILES.items()}[v.value]
 
     def autotune(self, P, steps=20):
-        """Time `steps` steps with each tile shape on the current state (which
-        is restored afterwards), keep the fastest and return its name."""
+        """Time `steps` steps with each named tile shape on the current state
+        (which is restored afterwards), set the fastest and return its name. What
+        an unset handle's kernels run is not among them."""
         p = P if isinstance(P, RnParams) else params_from_P(P)
         v = ctypes.c_int()
         _check(lib().rn_autotune(self.h, ctypes.byref(p), int(steps), ctypes.byref(v)))

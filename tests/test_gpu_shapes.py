@@ -404,6 +404,33 @@ def test_a_members_bits_do_not_depend_on_its_companions(rn, kind):
         g.close()
 
 
+def test_autotune_sets_the_shape_it_names(rn):
+    """After rn_autotune on a small unset handle the kernels run the shape it
+    returned: resized, the handle steps with the bits of one set to that name
+    (fast precision, where an unset handle's of the larger grid are others)."""
+    from rocket_nozzle_cfd_solver_b200 import configs
+    small, s = (rn.build_sim_setup(configs.viscous_plume(*sz)[0]) for sz in ((128, 48), (1024, 287)))
+    outs = []
+    g = rn.GPUSolver(small.Nx, small.Nr)
+    g.setGeometry(small.geo)
+    init = small.initialState()
+    g.setState(init["A"], init["B"])
+    chosen = g.autotune(small.P, steps=120)
+    assert g.tile == chosen
+    g.resize(s.Nx, s.Nr)
+    h = rn.GPUSolver(s.Nx, s.Nr)
+    h.setTile(chosen)
+    init = s.initialState()
+    for q in (g, h):
+        assert q.tile == chosen
+        q.setGeometry(s.geo)
+        q.setState(init["A"], init["B"])
+        q.step(40, s.P)
+        outs.append(q.readAll())
+        q.close()
+    assert np.array_equal(outs[0]["A"], outs[1]["A"]) and np.array_equal(outs[0]["B"], outs[1]["B"])
+
+
 def test_unset_name_follows_a_resize(rn):
     """An unset handle is named by its present grid's size, a set one as set."""
     g = rn.GPUSolver(128, 48)
