@@ -1369,7 +1369,7 @@ int rn_autotune(rn_handle h, const rn_params* P, int steps, int* chosen) {
     return toSave ? cudaMemcpyAsync(p, h->wmax, sizeof(unsigned) * 2, k, h->stream)
                   : cudaMemcpyAsync(h->wmax, p, sizeof(unsigned) * 2, k, h->stream);
   };
-  const int cur = h->cur, stepIdx = h->stepIdx, wslot = h->wslot, scur = h->scur;
+  const int cur = h->cur, stepIdx = h->stepIdx, wslot = h->wslot, scur = h->scur, s1last = h->s1last;
   const bool wvalid = h->wvalid;
   const long long stepCount = h->stepCount, launches = h->launches;
   const uint32_t head = h->head, seed = h->seed;
@@ -1396,7 +1396,7 @@ int rn_autotune(rn_handle h, const rn_params* P, int steps, int* chosen) {
     if (rc == RN_OK && e == cudaSuccess && ms < bestMs) { bestMs = ms; best = shape; }
     // restore the state the trial advanced
     if (e == cudaSuccess) e = copy_all(false);
-    h->cur = cur; h->stepIdx = stepIdx; h->wslot = wslot; h->scur = scur; h->wvalid = wvalid;
+    h->cur = cur; h->stepIdx = stepIdx; h->wslot = wslot; h->scur = scur; h->s1last = s1last; h->wvalid = wvalid;
     h->stepCount = stepCount; h->head = head; h->seed = seed;
     // the spray's deposit sums start each step at zero whatever parity it has
     if (e == cudaSuccess)

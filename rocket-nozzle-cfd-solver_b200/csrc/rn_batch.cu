@@ -859,7 +859,7 @@ int rn_batch_autotune(rn_batch b, int steps, int* chosen) {
   struct Saved {
     char* buf = nullptr;
     size_t state = 0, spray = 0;
-    int cur, stepIdx, wslot, scur;
+    int cur, stepIdx, wslot, scur, s1last;
     bool wvalid;
     long long stepCount;
     uint32_t head, seed;
@@ -878,7 +878,7 @@ int rn_batch_autotune(rn_batch b, int steps, int* chosen) {
     s.spray = inj ? sizeof(float4) * SPRAY_N * 6 : 0;
     cudaError_t e = cudaMalloc(&s.buf, s.state + s.spray + sizeof(float4) * 2 + sizeof(unsigned) * 2);
     if (e != cudaSuccess) { s.buf = nullptr; release(); return rn_record_cuda(e, "rn_batch_autotune: cudaMalloc"); }
-    s.cur = h->cur; s.stepIdx = h->stepIdx; s.wslot = h->wslot; s.scur = h->scur; s.wvalid = h->wvalid;
+    s.cur = h->cur; s.stepIdx = h->stepIdx; s.wslot = h->wslot; s.scur = h->scur; s.s1last = h->s1last; s.wvalid = h->wvalid;
     s.stepCount = h->stepCount; s.head = h->head; s.seed = h->seed;
   }
   auto copy_all = [&](bool toSave) -> cudaError_t {
@@ -896,7 +896,7 @@ int rn_batch_autotune(rn_batch b, int steps, int* chosen) {
         p += q.n;
       }
       if (!toSave) {
-        h->cur = s.cur; h->stepIdx = s.stepIdx; h->wslot = s.wslot; h->scur = s.scur; h->wvalid = s.wvalid;
+        h->cur = s.cur; h->stepIdx = s.stepIdx; h->wslot = s.wslot; h->scur = s.scur; h->s1last = s.s1last; h->wvalid = s.wvalid;
         h->stepCount = s.stepCount; h->head = s.head; h->seed = s.seed;
         // the spray's deposit sums start each step at zero whatever parity it has
         cudaError_t e = cudaMemsetAsync(h->acc, 0, sizeof(unsigned long long) * 8 * size_t(h->Nx) * h->Nr,

@@ -443,3 +443,35 @@ def test_unset_name_follows_a_resize(rn):
     g.resize(128, 48)
     assert g.tile == "16x8"
     g.close()
+
+
+@pytest.mark.parametrize("done", [0, 1, 2])
+@pytest.mark.parametrize("batched", [False, True])
+def test_autotune_leaves_the_turbulence_fields(rn, done, batched):
+    """The fields formed from the last step's stage-1 state (turbulence and
+    mixing rate) are the same before and after the trials of an autotuner, whose
+    steps are odd in number, on a spray handle that has taken no, an odd and an
+    even number of steps (the stage-1 slot alternates with the steps' parity)."""
+    from rocket_nozzle_cfd_solver_b200 import configs, solver
+    s = rn.build_sim_setup(dict(configs.injector_spray(192, 72)[0], startMode="burst"))
+    init = s.initialState()
+    g = rn.GPUSolver(s.Nx, s.Nr)
+    g.setGeometry(s.geo)
+    g.setState(init["A"], init["B"])
+    rn.GPUSpray(g).resize()
+    g.spray.setInjector(s.injector)
+    if done:
+        g.step(done, s.P)
+    specs = [solver.derived_spec(s, f) for f in (9, 13)]
+    before = [g.derived(sp, s.P).copy() for sp in specs]
+    if batched:
+        batch = rn.SolverBatch()
+        batch.add(g, s.P)
+        batch.autotune(steps=5)
+    else:
+        g.autotune(s.P, steps=5)
+    after = [g.derived(sp, s.P) for sp in specs]
+    assert all(np.array_equal(a, b) for a, b in zip(before, after))
+    if batched:
+        batch.close()
+    g.close()
