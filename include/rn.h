@@ -201,9 +201,9 @@ int rn_get_precision(rn_handle h, int* mode);
  * (or, while none is set, resized) handle is named RN_TILE_14x16 when the grid's
  * 14 x 16 tiles number at most 3 per SM (all resident at once), else
  * RN_TILE_16x15; until a shape is set its kernels may run another that suits the
- * grid's size better (10 x 10 on small grids, 16 x 16 where that saves a wave of
- * blocks) under that name. Setting a shape, that name too, makes them run the
- * shape named. rn_autotune times `steps` steps with each named shape on a copy
+ * grid's size better (10 x 10 on small grids, 16 x 16 where that takes clearly
+ * fewer tiles or a wave of blocks less) under that name. Setting a shape, that
+ * name too, makes them run the shape named. rn_autotune times `steps` steps with each named shape on a copy
  * of the handle's current state (the state, step info and spray ring are
  * restored afterwards), sets the fastest and returns it in *chosen; the shape of
  * an unset handle is not among them, and on small grids is faster than they

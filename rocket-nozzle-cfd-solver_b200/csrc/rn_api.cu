@@ -303,7 +303,7 @@ int rn_auto_shape(int Nx, int Nr, int numSMs) {
   if (tile_count(SHAPE_SMALL, Nx, Nr) <= 3 * numSMs) return SHAPE_SMALL;
   const int tile = rn_default_tile(Nx, Nr, numSMs);
   if (tile == RN_TILE_16x15 &&
-      prefer_16x16(tile_count(RN_TILE_16x16, Nx, Nr), tile_count(RN_TILE_16x15, Nx, Nr)))
+      prefer_16x16(tile_count(RN_TILE_16x16, Nx, Nr), tile_count(RN_TILE_16x15, Nx, Nr), numSMs))
     return RN_TILE_16x16;
   return tile;
 }

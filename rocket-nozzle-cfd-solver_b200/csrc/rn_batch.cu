@@ -516,7 +516,7 @@ int join_shape(rn_batch_t* b, rn_solver* h) {
       t16 += tile_count(RN_TILE_16x16, q->Nx, q->Nr);
       t15 += tile_count(RN_TILE_16x15, q->Nx, q->Nr);
     }
-    if (!b->longLists && prefer_16x16(t16, t15)) {
+    if (!b->longLists && prefer_16x16(t16, t15, b->numSMs)) {
       b->longLists = use_shape(b, RN_TILE_16x16) != RN_OK || rn_use_shape(h, RN_TILE_16x16) != RN_OK ||
                      h->maxX > XSMALL;
       for (const rn_solver* q : b->members) b->longLists |= q->maxX > XSMALL;

@@ -35,12 +35,25 @@ constexpr int SHAPE_SMALL = 5;
 inline int tile_count(int shape, int Nx, int Nr) {
   return ((Nx + TILE_TX[shape] - 1) / TILE_TX[shape]) * ((Nr + TILE_TY[shape] - 1) / TILE_TY[shape]);
 }
-// 16x16 in place of 16x15 where it needs clearly fewer tiles for the same grids
-// (heights that 15 divides badly): a 16x16 tile costs more than its 7 % of cells.
-// us per step, 16x15 / 16x16: viscous 1024x287 (1280 / 1152 tiles) 48.9 / 45.7,
-// 64 batched 128x48 (2048 / 1536) 103 / 92; 1024x384 (1664 / 1536) 59.1 / 65.8, 24
-// batched mixed grids (2224 / 2040 a set of four) 540 / 602.
-inline bool prefer_16x16(long long tiles16x16, long long tiles16x15) { return 11 * tiles16x16 <= 10 * tiles16x15; }
+// 16x16 in place of 16x15. A 16x16 tile costs 1.1 to 1.2 of a 16x15 one for 7 %
+// more cells (its 272 faces a direction take two passes of 256 threads), so it
+// has to save tiles or waves of resident blocks (4 an SM, 592 on 148 SMs):
+//   a wave of at most three. us per step, 16x15 / 16x16: viscous 640x224 (600 /
+//     560 tiles) 29.8 / 27.8, plain 22.9 / 20.6; presets of 1024x287 (1280 / 1152)
+//     47.6 / 45.5; 24 batched 128x48 (768 / 576) 48.2 / 38.0. At worst viscous
+//     1184x256 (1332 / 1184) 48.5 / 49.3. Of four: viscous 1400x320 (1936 / 1760)
+//     65.5 / 65.9, plain 50.1 / 50.9.
+//   a seventh of the tiles, beyond one wave: 64 batched 128x48 (2048 / 1536) 98.8 /
+//     88.5, 32 of 256x96 (3584 / 3072) 161 / 154, 32 of 203x77 (2496 / 2080) 116 /
+//     110. With less to save: viscous 640x288 (800 / 720) 33.3 / 36.3, 2048x512
+//     (4480 / 4096) 145 / 148, 24 batched mixed grids (13344 / 12240) 535 / 592;
+//     in one wave: viscous 512x256 (576 / 512) 25.4 / 27.4, 4 batched 128x48 (128 /
+//     96) 24.1 / 25.7.
+inline bool prefer_16x16(long long tiles16x16, long long tiles16x15, int numSMs) {
+  const long long resident = 4LL * numSMs;
+  const long long waves16 = (tiles16x16 + resident - 1) / resident, waves15 = (tiles16x15 + resident - 1) / resident;
+  return (waves16 < waves15 && waves15 <= 3) || (waves15 > 1 && 7 * tiles16x16 <= 6 * tiles16x15);
+}
 // A cell's class byte, in the row-pitched plane that the step kernels copy with
 // the halo (0 outside the grid). Almost all cells are uncut (99 % of the plume
 // and engine grids): their geometry is that of the grid, so the kernels form it

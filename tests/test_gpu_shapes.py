@@ -475,3 +475,21 @@ def test_autotune_leaves_the_turbulence_fields(rn, done, batched):
     if batched:
         batch.close()
     g.close()
+
+
+@pytest.mark.parametrize("kind,Nx,Nr", [("plain_small", 512, 192), ("plain_small", 640, 224), ("viscous_plume", 640, 224),
+                                        ("plain_small", 1024, 287), ("viscous_plume", 1024, 287),
+                                        ("plain_small", 4700, 64)])
+def test_larger_default_shapes_match_set_shapes(rn, kind, Nx, Nr):
+    """Unset handles beyond the 10x10 sizes, exact precision, against set 16x8
+    tiles: 14x16 with two to three blocks an SM, inviscid (both stage kernels
+    are dependent launches there); 16x16 by a wave saved (2 to 1, 3 to 2) and by
+    tiles saved; and, at viscous 1024x287, 16x15 again for its long lists."""
+    from rocket_nozzle_cfd_solver_b200 import configs
+    s = rn.build_sim_setup(getattr(configs, kind)(Nx, Nr)[0])
+    if (Nx, Nr) == (1024, 287):
+        assert (longest_list(s.geo["geoM"], Nx, Nr, 16, 16) > 4) == (kind == "viscous_plume")
+    calls = (1, 13, 4, 4, 15)
+    a, b = run(rn, s, None, calls), run(rn, s, "16x8", calls)
+    assert np.array_equal(a[0]["A"], b[0]["A"]) and np.array_equal(a[0]["B"], b[0]["B"])
+    assert np.array_equal(a[1], b[1])
