@@ -1363,9 +1363,11 @@ static bool step_kernel_attributes(K* kernel, size_t smem) {
 template <class T>
 static int init_tile() {
   const size_t ss = stage_smem_t<T>(MAXX), ps = fused_smem_t<T>(MAXX);
-  const bool ok = step_kernel_attributes(k_stage<T, 1>, ss) && step_kernel_attributes(k_stage<T, 2>, ss) &&
-                  step_kernel_attributes(k_stage2phys<T>, ps) && step_kernel_attributes(k_stage_batch<T, 1>, ss) &&
-                  step_kernel_attributes(k_stage_batch<T, 2>, ss) && step_kernel_attributes(k_stage2phys_batch<T>, ps);
+  bool ok = step_kernel_attributes(k_stage<T, 1>, ss) && step_kernel_attributes(k_stage<T, 2>, ss) &&
+            step_kernel_attributes(k_stage2phys<T>, ps);
+  if constexpr (T::ID < NTILES)                  // batches run the shapes that have names
+    ok = ok && step_kernel_attributes(k_stage_batch<T, 1>, ss) && step_kernel_attributes(k_stage_batch<T, 2>, ss) &&
+         step_kernel_attributes(k_stage2phys_batch<T>, ps);
   return ok ? 0 : -1;
 }
 // Raises the dynamic shared-memory limits of the stage and physics kernels to
@@ -1435,16 +1437,14 @@ void launch_stage2phys(const StageArgs& a, const PhysArgs& p, const rn_params& P
   else stage2phys_t<Tile0>(a, p, P, heavy, nHeavy, skip, s);
 }
 void launch_batch_stage1(const BatchInst* d, const int* bi, int nb, BatchPhase ph, int tile, cudaStream_t s) {
-  if (tile == 5) k_stage_batch<Tile5, 1><<<nb, Tile5::NT, stage_smem_t<Tile5>(ph.maxX), s>>>(d, bi, ph);
-  else if (tile == 4) k_stage_batch<Tile4, 1><<<nb, Tile4::NT, stage_smem_t<Tile4>(ph.maxX), s>>>(d, bi, ph);
+  if (tile == 4) k_stage_batch<Tile4, 1><<<nb, Tile4::NT, stage_smem_t<Tile4>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 3) k_stage_batch<Tile3, 1><<<nb, Tile3::NT, stage_smem_t<Tile3>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 2) k_stage_batch<Tile2, 1><<<nb, Tile2::NT, stage_smem_t<Tile2>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 1) k_stage_batch<Tile1, 1><<<nb, Tile1::NT, stage_smem_t<Tile1>(ph.maxX), s>>>(d, bi, ph);
   else k_stage_batch<Tile0, 1><<<nb, Tile0::NT, stage_smem_t<Tile0>(ph.maxX), s>>>(d, bi, ph);
 }
 void launch_batch_stage2(const BatchInst* d, const int* bi, int nb, BatchPhase ph, int tile, cudaStream_t s) {
-  if (tile == 5) k_stage_batch<Tile5, 2><<<nb, Tile5::NT, stage_smem_t<Tile5>(ph.maxX), s>>>(d, bi, ph);
-  else if (tile == 4) k_stage_batch<Tile4, 2><<<nb, Tile4::NT, stage_smem_t<Tile4>(ph.maxX), s>>>(d, bi, ph);
+  if (tile == 4) k_stage_batch<Tile4, 2><<<nb, Tile4::NT, stage_smem_t<Tile4>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 3) k_stage_batch<Tile3, 2><<<nb, Tile3::NT, stage_smem_t<Tile3>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 2) k_stage_batch<Tile2, 2><<<nb, Tile2::NT, stage_smem_t<Tile2>(ph.maxX), s>>>(d, bi, ph);
   else if (tile == 1) k_stage_batch<Tile1, 2><<<nb, Tile1::NT, stage_smem_t<Tile1>(ph.maxX), s>>>(d, bi, ph);
@@ -1465,8 +1465,7 @@ static void batch_stage2phys_t(const BatchInst* d, const int* bi, int nb, BatchP
 }
 void launch_batch_stage2phys(const BatchInst* d, const int* bi, int nb, BatchPhase ph, int tile, const int2* heavy,
                              int nHeavy, bool skip, cudaStream_t s) {
-  if (tile == 5) batch_stage2phys_t<Tile5>(d, bi, nb, ph, heavy, nHeavy, skip, s);
-  else if (tile == 4) batch_stage2phys_t<Tile4>(d, bi, nb, ph, heavy, nHeavy, skip, s);
+  if (tile == 4) batch_stage2phys_t<Tile4>(d, bi, nb, ph, heavy, nHeavy, skip, s);
   else if (tile == 3) batch_stage2phys_t<Tile3>(d, bi, nb, ph, heavy, nHeavy, skip, s);
   else if (tile == 2) batch_stage2phys_t<Tile2>(d, bi, nb, ph, heavy, nHeavy, skip, s);
   else if (tile == 1) batch_stage2phys_t<Tile1>(d, bi, nb, ph, heavy, nHeavy, skip, s);
