@@ -39,9 +39,11 @@ WORKLOAD = "viscous plume 512x192 (methalox gamma 1.2, T0 3500 K, p0 70 bar, bel
 # algorithmic HBM bytes per cell for each kernel kind (fused design): state
 # planes are 32 B per cell (A 16 + B 16), geometry 49 B (geoA, geoG, geoM 16
 # each + the class byte) in the 14x16 kernels, the class byte alone in the other
-# shapes (uncut cells' geometry is formed, not read); spray parcels 112 B each.
+# shapes (uncut cells' geometry is formed, not read); the spray apply reads the
+# class byte, the state and the step's four 8-byte deposit sums, clears the next
+# step's sums and writes the state; spray parcels 112 B each.
 STATE_BYTES = {"stage1": 32 + 32, "stage2": 32 + 32 + 32, "stage2_physics": 32 + 32 + 32,
-               "apply": 32 + 16 + 33 + 32, "reduce": 32 + 1}
+               "apply": 1 + 32 + 32 + 32 + 32, "reduce": 32 + 1}
 
 
 def bytes_per_cell(kind, tile):
@@ -64,15 +66,15 @@ def measured_peak():
         return 6650.0, "fallback"
 
 
-def profiled_traffic(kind):
-    """DRAM bytes per cell of a kernel from the committed ncu summary, if any."""
+def profiled_traffic(kind, tile):
+    """DRAM bytes per cell of a kernel with a tile shape from the committed ncu summary, if it has them."""
     path = os.path.join(ROOT, "profiles", "traffic_per_cell.txt")
     try:
         with open(path) as f:
             for line in f:
                 parts = line.split()
-                if len(parts) >= 2 and parts[0] == kind:
-                    return float(parts[1])
+                if len(parts) == 3 and parts[:2] == [tile, kind]:
+                    return float(parts[2])
     except OSError:
         pass
     return None
@@ -350,7 +352,7 @@ def run_ours(args, rank, world, local_rank):
     peak, peak_kind = measured_peak()
     bpc = bytes_per_cell(kind, tile_name)
     achieved = bpc * cells / (avg_ms * 1e-3) / 1e9 if bpc else None
-    traffic_pc = profiled_traffic(kind)
+    traffic_pc = profiled_traffic(kind, tile_name)
 
     def frac_of(t_ms):
         return bpc * cells / (t_ms * 1e-3) / 1e9 / peak if bpc else None

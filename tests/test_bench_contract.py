@@ -60,3 +60,16 @@ def test_clock_summary_keeps_the_timed_window():
     assert s["samples"] == 1 and s["sm_mhz"] == 1500.0 and s["reasons"] == ["sw_thermal_slowdown"]
     c.samples = []
     assert c.summary()["reasons"] == ["unsampled"]
+
+
+def test_traffic_is_that_of_the_kernel_and_tile():
+    """roofline.traffic takes the profiled bytes of the tile shape that ran;
+    a kernel moves about its algorithmic bytes at least (a third may still be in
+    L2 when it ends), and a shape that was not profiled has no figure."""
+    sys.path.insert(0, ROOT)
+    import bench
+    for tile in ("14x16", "16x15"):
+        for kind in ("stage1", "stage2_physics"):
+            assert bench.profiled_traffic(kind, tile) >= 0.65 * bench.bytes_per_cell(kind, tile), (kind, tile)
+    assert bench.profiled_traffic("stage1", "14x16") > 1.5 * bench.profiled_traffic("stage1", "16x15")
+    assert bench.profiled_traffic("stage1", "32x15") is None and bench.profiled_traffic("apply", "14x16") is None
