@@ -824,9 +824,11 @@ bool graph_at_start(const rn_solver* h, const StepGraph& g, bool inj) {
 // Relative cost of n steps through a graph of B steps: each replay (about 3 us
 // on the device between two graphs, measured), each remaining step launched
 // kernel by kernel (4 us of the host a kernel), and a share of instantiating
-// the graph's nodes. k = kernels per step.
+// the graph's nodes. k = kernels per step, two and two more with sprays (a split
+// grid's launch for its heavy tiles and the exact parcels' sort are left out:
+// both belong to steps of 50 us and more, where the length matters little).
 double graph_cost(int n, int B, int k) { return (n / B) * 3.0 + (n % B) * 4.0 * k + 2.0 * B * k; }
-constexpr int GRAPH_NODES = 24;   // most kernels captured in one graph
+constexpr int GRAPH_NODES = 24;   // most kernels in one graph, so counted
 int graph_steps(int n, int k) {
   int best = STEP_PERIOD;
   for (int B = STEP_PERIOD; B <= n && B * k <= GRAPH_NODES; B += STEP_PERIOD)

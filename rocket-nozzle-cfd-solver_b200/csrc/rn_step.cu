@@ -409,9 +409,12 @@ __device__ __forceinline__ void store_areas(const Grid& g, int x0, int y0, const
 // the normal are primitive slots b, b + d, b + 2d, b + 3d and its sensor cells
 // (k1 +- t, ij +- t of makeFluxShader, solver.js:133-259) b + d +- t and
 // b + 2d +- t: tile faces have (d, t) = (1, PX) (x) or (PX, 1) (r); a listed
-// member's faces live in its 5x5 block, with 5 in place of PX. One code path
-// for every face also makes the fast precision's contracted multiply-adds
-// round alike in every tile shape.
+// member's faces live in its 5x5 block, with 5 in place of PX. In exact
+// precision every tile shape gives the same bits. In fast precision the shapes
+// of 32 warps do among themselves (values below the smallest normal float
+// apart: flushed or not as an operation comes packed or alone); the WIDE ones,
+// which combine the Runge-Kutta stages and form vcell's differences otherwise,
+// agree with them to a few roundings.
 template <class T>
 __device__ __forceinline__ void inviscid_face(int k, bool dirR, int b, int d, int t, const rn_params& P,
                                               const float4* sW, const float4* sWb, float4* sF, float4* sY, float* sO,
